@@ -317,12 +317,21 @@ def pseudo_quantize_device(w, bits: int, groupsize: int, iters: int = 10):
     (reconstruction fp32 ``[N, K]``, quantized_w uint8 ``[N, K, q]``, w_scale fp32 ``[N, K/g, q]``,
     w_zero fp32 ``[N, K/g, 1]``) - the tensors ``HLQ.export`` takes (HLQ.py:207-208) and
     ``export_from_tensors`` turns into the exported arrays."""
+    import torch
     n, k = w.shape
     if k % groupsize:
         raise ValueError("in_channel must be a multiple of the group size")
-    blocks = w.contiguous().float().reshape(-1, groupsize)
-    scales, zeros = fit_alternating_device(blocks, bits, iters)
-    quantized = quantize_with_scales_device(blocks, scales, zeros)
-    recon = (quantized.float() * scales.unsqueeze(1)).sum(dim=2) + zeros.unsqueeze(1)
-    return (recon.reshape(n, k), quantized.reshape(n, k, bits), scales.reshape(n, k // groupsize, bits),
-            zeros.reshape(n, k // groupsize, 1))
+    if not w.is_cuda:
+        raise RuntimeError("pseudo_quantize_device runs on CUDA tensors only")
+    w = w.contiguous().float()
+    blocks = n * k // groupsize
+    recon = torch.empty((n, k), dtype=torch.float32, device=w.device)
+    quantized = torch.empty((n, k, bits), dtype=torch.uint8, device=w.device)
+    scales = torch.empty((n, k // groupsize, bits), dtype=torch.float32, device=w.device)
+    zeros = torch.empty((n, k // groupsize, 1), dtype=torch.float32, device=w.device)
+    with torch.cuda.device(w.device):
+        st = _lib.lib().hlq_pseudo_quantize_device(w.data_ptr(), recon.data_ptr(), quantized.data_ptr(),
+                                                   scales.data_ptr(), zeros.data_ptr(), blocks, groupsize, bits, iters,
+                                                   torch.cuda.current_stream(w.device).cuda_stream)
+    _lib.check(st, "hlq_pseudo_quantize_device")
+    return recon, quantized, scales, zeros

@@ -99,6 +99,13 @@ int hlq_quantize_with_scales_device(const float *d_w, const float *d_scales, con
 int hlq_fit_alternating_device(const float *d_w, float *d_scales, float *d_zeros, int64_t blocks, int g, int q,
                                int iters, void *stream);
 
+/* The fit, the assignment and the reconstruction of every block in one pass over the weights: scales and
+ * zeros as hlq_fit_alternating_device, quant (uint8 [blocks][g][q]) as hlq_quantize_with_scales_device of
+ * those, recon fp32 [blocks][g] = sum of the scales whose bit is set + zero.
+ * Replaces: pseudo_quantize_tensor(use_alternating_optimization=True), GPTQ/quant.py:185-213. */
+int hlq_pseudo_quantize_device(const float *d_w, float *d_recon, uint8_t *d_quant, float *d_scales, float *d_zeros,
+                               int64_t blocks, int g, int q, int iters, void *stream);
+
 /* ---- bit-plane packing -------------------------------------------------------------- */
 
 /* bits: uint8 [q][n][k] of 0/1  ->  packed: uint8 [q][n][k/8]; channel 8i+j goes to bit j
