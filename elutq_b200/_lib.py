@@ -6,6 +6,7 @@ module's ``lib()`` raises, and every operator of the package fails with it.
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 from ctypes import POINTER, c_char_p, c_float, c_int, c_int64, c_size_t, c_uint, c_void_p
 
@@ -137,6 +138,27 @@ HLQ_INPUT_PLAIN, HLQ_INPUT_GATED_SILU, HLQ_INPUT_ADD_RMSNORM = 0, 1, 2
 HLQ_KV_POSITION_MAJOR, HLQ_KV_HEAD_MAJOR = 0, 1
 
 _LIB = None
+_FAST = None
+
+
+class _FastCalls:
+    """The entry points a program calls per linear, through the CPython module `_hlq_call`."""
+
+    def __init__(self):
+        try:
+            from . import _hlq_call
+        except ImportError as e:
+            raise ImportError("elutq_b200/_hlq_call.so is missing: build it with `python -m elutq_b200.build`") from e
+        addr = lambda name: ctypes.cast(getattr(lib(), name), c_void_p).value  # noqa: E731
+        self.linear_forward = functools.partial(_hlq_call.linear_forward, addr("hlq_linear_forward_impl"))
+        self.group_forward = functools.partial(_hlq_call.group_forward, addr("hlq_group_forward"))
+
+
+def fast() -> _FastCalls:
+    global _FAST
+    if _FAST is None:
+        _FAST = _FastCalls()
+    return _FAST
 
 
 def lib() -> ctypes.CDLL:

@@ -8,6 +8,7 @@ the C ABI.  There is no CPU path: using these classes without a GPU raises.
 from __future__ import annotations
 
 import ctypes
+import functools
 from typing import Optional
 
 import numpy as np
@@ -17,6 +18,10 @@ from . import _lib
 from .format import ExportedLinear, SparsePlane, export_from_tensors, read_export_dir
 
 _DTYPES = {torch.float16: _lib.HLQ_F16, torch.bfloat16: _lib.HLQ_BF16, torch.float32: _lib.HLQ_F32}
+
+
+_ACT_DTYPES = {torch.float16: _lib.HLQ_F16, torch.bfloat16: _lib.HLQ_BF16}
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)   # current_stream(device).cuda_stream without the Stream object
 
 
 def _stream_ptr(device: torch.device) -> int:
@@ -42,6 +47,7 @@ class HLQWeight:
         info = _lib.WeightInfo()
         _lib.check(_lib.lib().hlq_weight_get_info(self._h, ctypes.byref(info)), "hlq_weight_get_info")
         self.info = info
+        self.shape_key = (info.in_channel, info.out_channel, info.bits, info.groupsize)
 
     # -- construction ------------------------------------------------------------------
     @classmethod
@@ -162,17 +168,10 @@ class Workspace:
     def __init__(self, nbytes: int, device):
         self.device = torch.device(device)
         self.buf = torch.empty(max(int(nbytes), 256), dtype=torch.uint8, device=self.device)
+        self.ptr, self.nbytes = self.buf.data_ptr(), self.buf.numel()
         with torch.cuda.device(self.device):
             _lib.check(_lib.lib().hlq_workspace_init(self.buf.data_ptr(), self.buf.numel(),
                                                      _stream_ptr(self.device)), "hlq_workspace_init")
-
-    @property
-    def ptr(self):
-        return self.buf.data_ptr()
-
-    @property
-    def nbytes(self):
-        return self.buf.numel()
 
     def kernel_status(self) -> int:
         """Status word left by the kernels (0 = fine); synchronizes the current stream."""
@@ -182,6 +181,7 @@ class Workspace:
         return v.value
 
 
+@functools.lru_cache(maxsize=4096)
 def workspace_bytes(m: int, k: int, n: int, bits: int, groupsize: int) -> int:
     return int(_lib.lib().hlq_workspace_bytes(m, k, n, bits, groupsize))
 
@@ -219,31 +219,38 @@ def linear_forward(x: torch.Tensor, weight: HLQWeight, workspace: Workspace,
     (arm_gemm.cpp:871-924): x is ``[m, k]`` (or ``[..., k]``), y ``[m, n]``, y is overwritten."""
     if not x.is_cuda:
         raise RuntimeError("HLQ linear runs on CUDA tensors only (no CPU path)")
-    i = weight.info
-    k, n = i.in_channel, i.out_channel
-    if x.shape[-1] != k:
-        raise ValueError(f"x has {x.shape[-1]} input channels, the weight expects {k}")
-    lead = x.shape[:-1]
-    x2 = x.reshape(-1, k)
-    if not x2.is_contiguous():
-        x2 = x2.contiguous()
-    if x2.dtype not in (torch.float16, torch.bfloat16):
+    k, n, bits, groupsize = weight.shape_key
+    shape = x.shape
+    if shape[-1] != k:
+        raise ValueError(f"x has {shape[-1]} input channels, the weight expects {k}")
+    xdt = _ACT_DTYPES.get(x.dtype)
+    if xdt is None:
         raise TypeError("activations must be float16 or bfloat16")
-    m = x2.shape[0]
-    odt = out_dtype or (out.dtype if out is not None else x2.dtype)
+    if not x.is_contiguous():
+        x = x.contiguous()
+    m = x.numel() // k
+    odt = out_dtype or (out.dtype if out is not None else x.dtype)
+    result = out
     if out is None:
-        out = torch.empty((m, n), dtype=odt, device=x.device)
+        result = out = torch.empty(shape[:-1] + (n,), dtype=odt, device=x.device)
     elif out.shape[-1] != n or out.numel() != m * n or not out.is_contiguous() or out.dtype != odt:
         raise ValueError("out must be a contiguous [m, n] tensor of the output dtype")
-    need = workspace_bytes(m, k, n, i.bits, i.groupsize)
+    else:
+        result = out.reshape(*shape[:-1], n)
+    need = workspace_bytes(m, k, n, bits, groupsize)
     if workspace.nbytes < need:
         raise ValueError(f"workspace holds {workspace.nbytes} bytes, {need} needed")
-    with torch.cuda.device(x.device):
-        st = _lib.lib().hlq_linear_forward_impl(
-            impl, m, k, n, x2.data_ptr(), _DTYPES[x2.dtype], out.data_ptr(), _DTYPES[odt],
-            workspace.ptr, workspace.nbytes, weight.handle, _stream_ptr(x.device))
-    _lib.check(st, "hlq_linear_forward")
-    return out.reshape(*lead, n)
+    dev = x.get_device()
+    args = (impl, m, k, n, x.data_ptr(), xdt, out.data_ptr(), _DTYPES[odt], workspace.ptr, workspace.nbytes,
+            weight.handle.value, _raw_stream(dev))
+    if torch.cuda.current_device() == dev:
+        st = _lib.fast().linear_forward(*args)
+    else:
+        with torch.cuda.device(dev):
+            st = _lib.fast().linear_forward(*args)
+    if st:
+        _lib.check(st, "hlq_linear_forward")
+    return result
 
 
 class HLQGroup:
@@ -258,7 +265,7 @@ class HLQGroup:
         with torch.cuda.device(self.device):
             _lib.check(_lib.lib().hlq_group_create(ctypes.byref(out), len(self.weights), arr, max_m),
                        "hlq_group_create")
-        self._h = out
+        self._h, self._addr = out, out.value
         self.max_m = max_m
         self._bound = None
 
@@ -285,8 +292,14 @@ class HLQGroup:
         self._bound = (list(xs), list(ys))    # keeps the tensors alive
 
     def forward(self, m: int = 1):
-        with torch.cuda.device(self.device):
-            _lib.check(_lib.lib().hlq_group_forward(self._h, m, _stream_ptr(self.device)), "hlq_group_forward")
+        dev = self.device.index
+        if torch.cuda.current_device() == dev:
+            st = _lib.fast().group_forward(self._addr, m, _raw_stream(dev))
+        else:
+            with torch.cuda.device(dev):
+                st = _lib.fast().group_forward(self._addr, m, _raw_stream(dev))
+        if st:
+            _lib.check(st, "hlq_group_forward")
         return self._bound[1]
 
     def kernel_status(self) -> int:
@@ -308,7 +321,7 @@ class HLQGroup:
     def free(self):
         if self._h is not None:
             _lib.lib().hlq_group_free(self._h)
-            self._h = None
+            self._h = self._addr = None
 
     def __del__(self):
         try:
