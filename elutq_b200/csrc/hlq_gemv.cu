@@ -60,7 +60,7 @@ constexpr int kConsumers = kConsumerWarps * 32;
 constexpr int kFinalizers = kFinalWarps * 32;
 constexpr int kThreads = kConsumers + kFinalizers;
 constexpr uint32_t kTableBytes = 65536;
-constexpr uint32_t kAuxBytes = 8192;
+constexpr uint32_t kAuxBytes = 10240;     // a multiple of the 1 KB the shared window starts on
 
 // named barriers (0 is __syncthreads)
 constexpr int kBarConsumers = 1;   // 512 consumer threads
@@ -81,9 +81,48 @@ constexpr uint32_t kAuxX2 = 4096;      // two-row passes: 2 slots x 2 rows x 512
 constexpr uint32_t kAuxGamma = 6144;   // input transform: 2 slots x 512 RMSNorm weights
 constexpr uint32_t kAuxTp = 2560;      // copy of the TpDev of a fused all-reduce (<= 256 bytes)
 constexpr uint32_t kAuxXsum2 = 2816;   // two-row passes: 2 x 16 group sums
+constexpr int kPub = 4;                // counter updates a finalizer thread keeps in flight
+constexpr uint32_t kAuxList = 8192;    // finished blocks of a round of counter updates (16-bit offsets)
+constexpr uint32_t kAuxCount = kAuxList + kFinalizers * kPub * 2;   // how many there are
+constexpr uint32_t kAuxCur = kAuxCount + 16;                       // the segment the finalizers work on
+static_assert(kAuxCur + kAuxSegSlot <= kAuxBytes && sizeof(Seg) % 4 == 0 && sizeof(Seg) / 4 <= kFinalizers, "aux area");
 static_assert(sizeof(TpDev) <= 256, "TpDev must fit its slot");
 static_assert(sizeof(Seg) <= kAuxSegSlot, "Seg must fit its slot");
 static_assert(kAuxGamma + 2048 <= kAuxBytes, "aux area");
+
+// Four consecutive accumulators, read around L1 (a workspace off the 16-byte grid: one by one).
+__device__ __forceinline__ float4 load_acc4(const float *p, bool vec) {
+    if (vec) return __ldcg((const float4 *)p);
+    return make_float4(ldcg_f32(p), ldcg_f32(p + 1), ldcg_f32(p + 2), ldcg_f32(p + 3));
+}
+__device__ __forceinline__ void clear_acc4(float *p, bool vec) {
+    if (vec) *(float4 *)p = make_float4(0.f, 0.f, 0.f, 0.f);
+    else p[0] = p[1] = p[2] = p[3] = 0.f;
+}
+// Outputs of rows row .. row + 3 (those below n) plus the bias.
+__device__ __forceinline__ void store_y4(const Seg &sg, long long base, int row, const float4 &v) {
+    float o[4] = {v.x, v.y, v.z, v.w};
+    if (sg.bias)
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            if (row + e < sg.n) o[e] += __half2float(__ushort_as_half(sg.bias[row + e]));
+    unsigned char *dst = (unsigned char *)sg.y + 2 * (base + row);
+    if (sg.y_dtype != HLQ_F32 && row + 4 <= sg.n && !((uintptr_t)dst & 7)) {
+        uint2 pk;
+        if (sg.y_dtype == HLQ_F16) {
+            const __half2 a = __floats2half2_rn(o[0], o[1]), b = __floats2half2_rn(o[2], o[3]);
+            pk = make_uint2(*(const uint32_t *)&a, *(const uint32_t *)&b);
+        } else {
+            const __nv_bfloat162 a = __floats2bfloat162_rn(o[0], o[1]), b = __floats2bfloat162_rn(o[2], o[3]);
+            pk = make_uint2(*(const uint32_t *)&a, *(const uint32_t *)&b);
+        }
+        *(uint2 *)dst = pk;
+    } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            if (row + e < sg.n) store_y(sg.y, base + row + e, o[e], sg.y_dtype);
+    }
+}
 
 // R = rows of x one pass serves: 1, or 2 with half2 table entries {row, row + 1}.
 // XOP: the instantiation that applies the jobs' input transforms (one-row passes only), kept
@@ -126,6 +165,8 @@ __global__ void __launch_bounds__(kThreads, 1) lut8_gemv_kernel(const __grid_con
     if (warp >= kConsumerWarps) {
         // =========================== finalizer warps ======================================
         const int fw = warp - kConsumerWarps, ftid = tid - kConsumers;
+        uint16_t *list = (uint16_t *)(aux + kAuxList);
+        int *ndone = (int *)(aux + kAuxCount);
         Walker wk;
         bool waited = false;
         auto emit = [&](int slot) {   // control warp only
@@ -180,19 +221,7 @@ __global__ void __launch_bounds__(kThreads, 1) lut8_gemv_kernel(const __grid_con
         // (the descriptor is copied to shared memory once: it is read for every block)
         const TpDev *tp = nullptr;
         unsigned epoch = 0, par = 0;
-        Seg last_sg;
-        last_sg.live = 0;
         if (a.tp) {
-            // the second phase needs the (single) job's output even in a CTA whose unit range
-            // holds no duo
-            const Job &jb = a.single;
-            last_sg.live = 1;
-            last_sg.y = jb.y;
-            last_sg.y_base = (long long)mrow * jb.n;
-            last_sg.n = jb.n;
-            last_sg.y_dtype = jb.y_dtype;
-            last_sg.mrow = mrow;
-            last_sg.blocks = jb.blocks;
             uint32_t *dst = (uint32_t *)(aux + kAuxTp);
             const uint32_t *src = (const uint32_t *)a.tp;
             for (int i = ftid; i < (int)(sizeof(TpDev) / 4); i += kFinalizers) dst[i] = __ldg(src + i);
@@ -204,16 +233,19 @@ __global__ void __launch_bounds__(kThreads, 1) lut8_gemv_kernel(const __grid_con
         for (int i = 0;; ++i) {
             const int slot = i & 1;
             const bool have = mbar_wait_bounded(mb_desc + 8 * slot, (i >> 1) & 1, fail, spin);
-            const Seg sg = ring[slot];
-            if (!have || !sg.live) break;     // no descriptor: nothing may be read from the ring slot
-            last_sg = sg;
+            if (!have || !ring[slot].live) break;     // no descriptor: nothing may be read from the ring slot
             named_bar_sync_dyn(kBarSegDone + slot, kThreads);      // consumers are done with it
-            named_bar_sync<kBarFinalizers, kFinalizers>();         // every finalizer holds its copy
+            // a copy in shared memory for the finalizers (in registers it cost every warp of the kernel
+            // 200 bytes of local memory): the ring slot is free for segment i + 2
+            if (ftid < (int)(sizeof(Seg) / 4)) ((uint32_t *)(aux + kAuxCur))[ftid] = ((const uint32_t *)&ring[slot])[ftid];
+            if (ftid == 0) *ndone = 0;
+            named_bar_sync<kBarFinalizers, kFinalizers>();
+            const Seg &sg = *(const Seg *)(aux + kAuxCur);
             if (fw == 0) emit(slot);                               // segment i + 2
             // publish: count finished duos per 32-row block; whoever completes a block sums it
             const int bfirst = sg.duo_a >> 1, blast = (sg.duo_b - 1) >> 1;
             const unsigned total = (unsigned)sg.slices * 2u;
-            constexpr int kPub = 4;      // counter updates a thread keeps in flight
+            const bool vec = ((uintptr_t)sg.acc & 15) == 0;
             for (int b0 = bfirst; b0 <= blast; b0 += kFinalizers * kPub) {
                 unsigned minebits = 0;
                 if (b0 + ftid <= blast) __threadfence();
@@ -227,69 +259,84 @@ __global__ void __launch_bounds__(kThreads, 1) lut8_gemv_kernel(const __grid_con
                         minebits |= (old + cnt == total ? 1u : 0u) << i;
                     }
                 }
-#pragma unroll 1
-                for (int i = 0; i < kPub; ++i) {
-                const int blk = b0 + i * kFinalizers + ftid;
-                unsigned mask = __ballot_sync(0xffffffffu, (minebits >> i) & 1u);
-                if (mask) __threadfence();
-                // lane = row of a finished block; several blocks per round trip
-                while (mask) {
-                    float v[8], v2[R == 2 ? 8 : 1];
-                    int rows[8];
-                    unsigned mm = mask;
+                // The finished blocks of all finalizers in one list, which the 128 threads then take
+                // four rows at a time with kQuads reads in flight each.  The CTA whose segment ends last
+                // finishes nearly all blocks its segment covers (up to 448 in a Llama-3-8B gate
+                // projection), so this is the tail of the launch: with a warp reading eight blocks, one
+                // row a lane, it took 25 us of 70 for four layers in one launch (now 58) and 16 us of
+                // 79 for a 128256x4096 head at 4 bits (now 73).  Eight reads in flight instead of four
+                // spill registers and are no faster.
+                if (minebits) {
+                    __threadfence();
+                    int at = atomicAdd(ndone, __popc(minebits));
 #pragma unroll
-                    for (int b = 0; b < 8; ++b) {
-                        rows[b] = -1;
-                        if (mm) {
-                            const int src_lane = __ffs(mm) - 1;
-                            mm &= mm - 1;
-                            rows[b] = __shfl_sync(0xffffffffu, blk, src_lane) * kBlockRows + lane;
-                            v[b] = ldcg_f32(sg.acc + rows[b]);
-                            if constexpr (R == 2) v2[b] = ldcg_f32(sg.acc + sg.np + rows[b]);
-                        }
-                    }
-#pragma unroll
-                    for (int b = 0; b < 8; ++b) {
-                        if (rows[b] >= 0) {
-                            sg.acc[rows[b]] = 0.f;
-                            float o = v[b];
-                            if (sg.bias && rows[b] < sg.n) o += __half2float(__ushort_as_half(sg.bias[rows[b]]));
-                            if constexpr (R == 2) {       // the second row of x of this pass
-                                sg.acc[sg.np + rows[b]] = 0.f;
-                                float o2 = v2[b];
-                                if (sg.bias && rows[b] < sg.n) o2 += __half2float(__ushort_as_half(sg.bias[rows[b]]));
-                                if (rows[b] < sg.n) store_y(sg.y, sg.y_base + sg.n + rows[b], o2, sg.y_dtype);
-                            }
-                            if (!tp) {
-                                if (rows[b] < sg.n) store_y(sg.y, sg.y_base + rows[b], o, sg.y_dtype);
-                            } else {
-                                // push this rank's sum of the block to every rank (itself included)
-                                const long long slot_row =
-                                    (((long long)par * tp->world + tp->rank) * tp->max_m + sg.mrow) * tp->np_cap + rows[b];
-                                for (int p = 0; p < tp->world; ++p)
-                                    st_relaxed_sys_b64(tp->recv[p] + slot_row, __float_as_uint(o), epoch);
-                            }
-                            if (lane == 0) sg.counters[rows[b] / kBlockRows] = 0;
-                        }
-                    }
-                    mask = mm;
+                    for (int i = 0; i < kPub; ++i)
+                        if (minebits >> i & 1u) list[at++] = (uint16_t)(i * kFinalizers + ftid);
                 }
+                named_bar_sync<kBarFinalizers, kFinalizers>();
+                const int quads = *ndone * (kBlockRows / 4);
+                constexpr int kQuads = R == 2 ? 2 : 4;
+#pragma unroll 1
+                for (int q0 = ftid; q0 < quads; q0 += kFinalizers * kQuads) {
+                    float4 v[kQuads], v2[R == 2 ? kQuads : 1];
+                    int rows[kQuads];
+#pragma unroll
+                    for (int b = 0; b < kQuads; ++b) {
+                        const int qd = q0 + b * kFinalizers;
+                        rows[b] = -1;
+                        if (qd < quads) {
+                            rows[b] = (b0 + list[qd / (kBlockRows / 4)]) * kBlockRows + 4 * (qd % (kBlockRows / 4));
+                            v[b] = load_acc4(sg.acc + rows[b], vec);
+                            if constexpr (R == 2) v2[b] = load_acc4(sg.acc + sg.np + rows[b], vec);
+                        }
+                    }
+#pragma unroll
+                    for (int b = 0; b < kQuads; ++b) {
+                        if (rows[b] < 0) continue;
+                        clear_acc4(sg.acc + rows[b], vec);
+                        if constexpr (R == 2) {       // the second row of x of this pass
+                            clear_acc4(sg.acc + sg.np + rows[b], vec);
+                            store_y4(sg, sg.y_base + sg.n, rows[b], v2[b]);
+                        }
+                        if (!tp) {
+                            store_y4(sg, sg.y_base, rows[b], v[b]);
+                        } else {
+                            // push this rank's sum of the rows to every rank (itself included)
+                            const float o[4] = {v[b].x, v[b].y, v[b].z, v[b].w};
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) {
+                                const int row = rows[b] + e;
+                                const float bias = sg.bias && row < sg.n ? __half2float(__ushort_as_half(sg.bias[row])) : 0.f;
+                                const long long slot_row =
+                                    (((long long)par * tp->world + tp->rank) * tp->max_m + sg.mrow) * tp->np_cap + row;
+                                for (int p = 0; p < tp->world; ++p)
+                                    st_relaxed_sys_b64(tp->recv[p] + slot_row, __float_as_uint(o[e] + bias), epoch);
+                            }
+                        }
+                        if (rows[b] % kBlockRows == 0) sg.counters[rows[b] / kBlockRows] = 0;
+                    }
+                }
+                if (b0 + kFinalizers * kPub <= blast) {        // another round: the list is empty again
+                    named_bar_sync<kBarFinalizers, kFinalizers>();
+                    if (ftid == 0) *ndone = 0;
+                    named_bar_sync<kBarFinalizers, kFinalizers>();
                 }
             }
         }
-        if (tp && last_sg.live) {
+        if (tp) {
             // Second phase of the fused all-reduce.  Pushing never waits; summing is split
             // statically over the CTAs: poll every rank's slot of a row until it carries this
             // launch's number, add the ranks' sums in rank order, write y.
-            const Seg &sg = last_sg;
+            // The (single) job's output is known to a CTA whose unit range holds no duo, too.
+            const Job &jb = a.single;
             const int nwarps = gridDim.x * kFinalWarps;
-            for (int blk = blockIdx.x * kFinalWarps + fw; blk < sg.blocks; blk += nwarps) {
+            for (int blk = blockIdx.x * kFinalWarps + fw; blk < jb.blocks; blk += nwarps) {
                 const int row = blk * kBlockRows + lane;
                 float sum = 0.f;
                 bool ok = true;
                 for (int src = 0; src < tp->world; ++src) {
                     const unsigned long long *slot =
-                        tp->recv[tp->rank] + (((long long)par * tp->world + src) * tp->max_m + sg.mrow) * tp->np_cap + row;
+                        tp->recv[tp->rank] + (((long long)par * tp->world + src) * tp->max_m + mrow) * tp->np_cap + row;
                     unsigned long long v = ld_relaxed_sys_b64(slot);
                     // a peer that never arrives: the first wait that runs out ends all later ones
                     const int lim = *fail ? 0 : spin;
@@ -301,11 +348,11 @@ __global__ void __launch_bounds__(kThreads, 1) lut8_gemv_kernel(const __grid_con
                     sum += __uint_as_float((uint32_t)v);
                 }
                 if (!ok) *fail = 1;
-                if (row < sg.n) store_y(sg.y, sg.y_base + row, sum, sg.y_dtype);
+                if (row < jb.n) store_y(jb.y, (long long)mrow * jb.n + row, sum, jb.y_dtype);
                 __syncwarp();
                 if (lane == 0) {
                     const unsigned old = atomicAdd(tp->done, 1u);
-                    if (old + 1u == (unsigned)sg.blocks * gridDim.y) {     // last block of the launch
+                    if (old + 1u == (unsigned)jb.blocks * gridDim.y) {     // last block of the launch
                         *tp->done = 0u;
                         __threadfence();
                         *tp->seq = epoch;
