@@ -66,6 +66,7 @@ constexpr uint32_t kAuxBytes = 10240;     // a multiple of the 1 KB the shared w
 constexpr int kBarConsumers = 1;   // 512 consumer threads
 constexpr int kBarSegDone = 2;     // +slot: consumers arrive, finalizers sync (640)
 constexpr int kBarFinalizers = 6;  // 128 finalizer threads
+constexpr int kBarTail = 7;        // everyone: the last segment's finished blocks are listed
 
 // aux region layout (bytes from its start)
 constexpr uint32_t kAuxX = 0;          // 2 x 512 16-bit activations
@@ -121,6 +122,59 @@ __device__ __forceinline__ void store_y4(const Seg &sg, long long base, int row,
 #pragma unroll
         for (int e = 0; e < 4; ++e)
             if (row + e < sg.n) store_y(sg.y, base + row + e, o[e], sg.y_dtype);
+    }
+}
+
+// The listed finished blocks of a segment (offsets from block b0): outputs from their accumulators, which
+// are cleared, with the blocks' counters, for the next launch.  `nthreads` threads take four rows at a time,
+// four reads in flight each.  tp: the sums go to every rank's slots instead (fused all-reduce).
+// A function of its own with a rolled loop: the streaming loop keeps its registers, and the code, cold
+// when a CTA gets here, is short.
+template <int R>
+__device__ __noinline__ void finish_blocks(const Seg &sg, const uint16_t *list, int count, int b0, int t, int nthreads,
+                                           const TpDev *tp, unsigned par, unsigned epoch) {
+    const bool vec = ((uintptr_t)sg.acc & 15) == 0;
+    const int quads = count * (kBlockRows / 4);
+    constexpr int kQuads = 4 / R;
+#pragma unroll 1
+    for (int q0 = t; q0 < quads; q0 += nthreads * kQuads) {
+        float4 v[kQuads][R];
+#pragma unroll
+        for (int b = 0; b < kQuads; ++b) {
+            const int qd = q0 + b * nthreads;
+            if (qd >= quads) break;
+            const int row = (b0 + list[qd / (kBlockRows / 4)]) * kBlockRows + 4 * (qd % (kBlockRows / 4));
+#pragma unroll
+            for (int rr = 0; rr < R; ++rr) v[b][rr] = load_acc4(sg.acc + rr * sg.np + row, vec);
+        }
+#pragma unroll 1
+        for (int b = 0; b < kQuads; ++b) {
+            const int qd = q0 + b * nthreads;
+            if (qd >= quads) break;
+            const int row = (b0 + list[qd / (kBlockRows / 4)]) * kBlockRows + 4 * (qd % (kBlockRows / 4));
+            float4 f[R];
+#pragma unroll
+            for (int rr = 0; rr < R; ++rr) {
+                f[rr] = v[0][rr];
+#pragma unroll
+                for (int w = 0; w + 1 < kQuads; ++w) v[w][rr] = v[w + 1][rr];
+                clear_acc4(sg.acc + rr * sg.np + row, vec);
+                if (rr || !tp) store_y4(sg, sg.y_base + (long long)rr * sg.n, row, f[rr]);
+            }
+            if (tp) {
+                // push this rank's sum of the rows to every rank (itself included)
+                const float o[4] = {f[0].x, f[0].y, f[0].z, f[0].w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const float bias = sg.bias && row + e < sg.n ? __half2float(__ushort_as_half(sg.bias[row + e])) : 0.f;
+                    const long long slot_row =
+                        (((long long)par * tp->world + tp->rank) * tp->max_m + sg.mrow) * tp->np_cap + row + e;
+                    for (int p = 0; p < tp->world; ++p)
+                        st_relaxed_sys_b64(tp->recv[p] + slot_row, __float_as_uint(o[e] + bias), epoch);
+                }
+            }
+            if (row % kBlockRows == 0) sg.counters[row / kBlockRows] = 0;
+        }
     }
 }
 
@@ -245,7 +299,13 @@ __global__ void __launch_bounds__(kThreads, 1) lut8_gemv_kernel(const __grid_con
             // publish: count finished duos per 32-row block; whoever completes a block sums it
             const int bfirst = sg.duo_a >> 1, blast = (sg.duo_b - 1) >> 1;
             const unsigned total = (unsigned)sg.slices * 2u;
-            const bool vec = ((uintptr_t)sg.acc & 15) == 0;
+            // after the last segment the consumers have nothing left to stream and take their share of the list
+            const bool last = mbar_wait_bounded(mb_desc + 8 * (slot ^ 1), ((i + 1) >> 1) & 1, fail, spin) &&
+                              !ring[slot ^ 1].live && !tp;
+            auto round_barrier = [&]() {
+                if (last) named_bar_sync<kBarTail, kThreads>();
+                else named_bar_sync<kBarFinalizers, kFinalizers>();
+            };
             for (int b0 = bfirst; b0 <= blast; b0 += kFinalizers * kPub) {
                 unsigned minebits = 0;
                 if (b0 + ftid <= blast) __threadfence();
@@ -259,13 +319,12 @@ __global__ void __launch_bounds__(kThreads, 1) lut8_gemv_kernel(const __grid_con
                         minebits |= (old + cnt == total ? 1u : 0u) << i;
                     }
                 }
-                // The finished blocks of all finalizers in one list, which the 128 threads then take
-                // four rows at a time with kQuads reads in flight each.  The CTA whose segment ends last
+                // The finished blocks of all finalizers in one list.  The CTA whose segment ends last
                 // finishes nearly all blocks its segment covers (up to 448 in a Llama-3-8B gate
                 // projection), so this is the tail of the launch: with a warp reading eight blocks, one
-                // row a lane, it took 25 us of 70 for four layers in one launch (now 58) and 16 us of
-                // 79 for a 128256x4096 head at 4 bits (now 73).  Eight reads in flight instead of four
-                // spill registers and are no faster.
+                // row a lane, it took 25 us of 70 for four layers in one launch and 16 us of 79 for a
+                // 128256x4096 head at 4 bits.  Four rows a thread: 58 and 73 us in all; with the
+                // consumers' help after the last segment 55 and 71.5.
                 if (minebits) {
                     __threadfence();
                     int at = atomicAdd(ndone, __popc(minebits));
@@ -273,51 +332,11 @@ __global__ void __launch_bounds__(kThreads, 1) lut8_gemv_kernel(const __grid_con
                     for (int i = 0; i < kPub; ++i)
                         if (minebits >> i & 1u) list[at++] = (uint16_t)(i * kFinalizers + ftid);
                 }
-                named_bar_sync<kBarFinalizers, kFinalizers>();
-                const int quads = *ndone * (kBlockRows / 4);
-                constexpr int kQuads = R == 2 ? 2 : 4;
-#pragma unroll 1
-                for (int q0 = ftid; q0 < quads; q0 += kFinalizers * kQuads) {
-                    float4 v[kQuads], v2[R == 2 ? kQuads : 1];
-                    int rows[kQuads];
-#pragma unroll
-                    for (int b = 0; b < kQuads; ++b) {
-                        const int qd = q0 + b * kFinalizers;
-                        rows[b] = -1;
-                        if (qd < quads) {
-                            rows[b] = (b0 + list[qd / (kBlockRows / 4)]) * kBlockRows + 4 * (qd % (kBlockRows / 4));
-                            v[b] = load_acc4(sg.acc + rows[b], vec);
-                            if constexpr (R == 2) v2[b] = load_acc4(sg.acc + sg.np + rows[b], vec);
-                        }
-                    }
-#pragma unroll
-                    for (int b = 0; b < kQuads; ++b) {
-                        if (rows[b] < 0) continue;
-                        clear_acc4(sg.acc + rows[b], vec);
-                        if constexpr (R == 2) {       // the second row of x of this pass
-                            clear_acc4(sg.acc + sg.np + rows[b], vec);
-                            store_y4(sg, sg.y_base + sg.n, rows[b], v2[b]);
-                        }
-                        if (!tp) {
-                            store_y4(sg, sg.y_base, rows[b], v[b]);
-                        } else {
-                            // push this rank's sum of the rows to every rank (itself included)
-                            const float o[4] = {v[b].x, v[b].y, v[b].z, v[b].w};
-#pragma unroll
-                            for (int e = 0; e < 4; ++e) {
-                                const int row = rows[b] + e;
-                                const float bias = sg.bias && row < sg.n ? __half2float(__ushort_as_half(sg.bias[row])) : 0.f;
-                                const long long slot_row =
-                                    (((long long)par * tp->world + tp->rank) * tp->max_m + sg.mrow) * tp->np_cap + row;
-                                for (int p = 0; p < tp->world; ++p)
-                                    st_relaxed_sys_b64(tp->recv[p] + slot_row, __float_as_uint(o[e] + bias), epoch);
-                            }
-                        }
-                        if (rows[b] % kBlockRows == 0) sg.counters[rows[b] / kBlockRows] = 0;
-                    }
-                }
+                round_barrier();
+                finish_blocks<R>(sg, list, *ndone, b0, last ? kConsumers + ftid : ftid, last ? kThreads : kFinalizers, tp, par,
+                                 epoch);
                 if (b0 + kFinalizers * kPub <= blast) {        // another round: the list is empty again
-                    named_bar_sync<kBarFinalizers, kFinalizers>();
+                    round_barrier();
                     if (ftid == 0) *ndone = 0;
                     named_bar_sync<kBarFinalizers, kFinalizers>();
                 }
@@ -380,7 +399,7 @@ __global__ void __launch_bounds__(kThreads, 1) lut8_gemv_kernel(const __grid_con
     const uint8_t *pl;
     const uint16_t *mp;
     float *prow;
-    int d, dend, x_dtype, acc_stride = 0;
+    int d, d_first = 0, dend, x_dtype, acc_stride = 0;
     // input transform of the current segment's job
     const Job *cur_job = nullptr, *rms_job = nullptr;
     int cur_slice = 0, cur_xop = 0, cur_k = 0;
@@ -389,6 +408,7 @@ __global__ void __launch_bounds__(kThreads, 1) lut8_gemv_kernel(const __grid_con
 
     auto open_segment = [&](const Seg &sg) {
         d = sg.duo_a + warp;
+        d_first = sg.duo_a;
         dend = sg.duo_b;
         x_dtype = sg.x_dtype;
         acc_stride = sg.np;
@@ -588,7 +608,19 @@ __global__ void __launch_bounds__(kThreads, 1) lut8_gemv_kernel(const __grid_con
         const bool more = have && nx.live;
         if (more) open_segment(nx);
         named_bar_arrive_dyn(kBarSegDone + slot, kThreads);
-        if (!more) break;
+        if (!more) {
+            // the finalizers list the blocks this segment finished, everyone turns them into outputs
+            if (have && !a.tp) {
+                const Seg &sg = *(const Seg *)(aux + kAuxCur);
+                for (int b0 = d_first >> 1; b0 <= (dend - 1) >> 1; b0 += kFinalizers * kPub) {
+                    if (b0 != d_first >> 1) named_bar_sync<kBarTail, kThreads>();      // the round before is done
+                    named_bar_sync<kBarTail, kThreads>();
+                    finish_blocks<R>(sg, (const uint16_t *)(aux + kAuxList), *(const int *)(aux + kAuxCount), b0, tid, kThreads,
+                                     nullptr, 0u, 0u);
+                }
+            }
+            break;
+        }
     }
 }
 
