@@ -27,11 +27,13 @@
 //   * fp32 accumulators of a duo (16 rows x up to 16 rows of x) are added to global accumulators
 //     [output row][row of x] with 128-bit reductions; completion counters per block of 32 rows
 //     and the finalizing pass are those of the LUT kernel, run by one warp.
-//   * At a CTA's two ends that warp is not alone: all consumers arrange the first segment's
-//     activations, and all warps take the finished blocks of the last segment in turn.  A call of one
-//     linear is little else than these two ends (4096x4096, 4 rows: 2.1 us arranging and 4.6 us from the
-//     last weight to the last output, of 11 us, with one warp doing both).  Seven projections of a
-//     Llama-3-8B layer, 3 bits, 4 rows, call by call: 110.8 -> 83.0 us.
+//   * That warp has no time for more than counting: the consumers arrange the first segment's
+//     activations, and they turn the blocks a segment finished into outputs after the next one (all
+//     warps after the last).  A call of one linear is little else than its two ends (4096x4096, 4 rows:
+//     2.1 us arranging and 4.6 us from the last weight to the last output, of 11 us, with one warp doing
+//     both), and in a group the CTAs that finished many blocks were 20 us behind the others.  Seven
+//     projections of a Llama-3-8B layer, 3 bits, 4 rows, call by call: 110.8 -> 84 us; four layers in
+//     one launch, 16 rows: 189.9 -> 171 us.
 //
 // What bounds it: the integer pipe.  A sub-partition issues one prmt / lop3 / shf every two cycles,
 // and a duo costs each lane about 540 of them (256 table permutes, 160 for the selectors, the
@@ -66,26 +68,26 @@ constexpr int kBmBarConsumers = 4;           // the consumers have arranged the 
 // same unit) read 16 different 8-byte bank slots.
 constexpr uint32_t kBmRowStride = 1056, kBmQuarterStride = 264;
 constexpr uint32_t kBmBBytes = 16 * kBmRowStride;    // one buffer: 16 rows of x
-constexpr int kBmStageBlocks = 16;                   // blocks of 32 rows whose accumulators are staged at once
 
 // shared memory (bytes from the 1 KB-aligned base)
 constexpr uint32_t kBmB = 0;                                   // 2 buffers of fragment-ordered activations
 constexpr uint32_t kBmRaw = 2 * kBmBBytes;                     // 2 slots x [16][512] 16-bit activations as they come
-constexpr uint32_t kBmStage = kBmRaw + 2 * 16384;              // accumulators of finished blocks (up to 2 KB each)
-constexpr int kBmListBlocks = 128;                             // candidates looked at per round of counter updates
-constexpr uint32_t kBmList = kBmStage + kBmStageBlocks * 2048; // finished blocks among them
-constexpr uint32_t kBmSeg = kBmList + kBmListBlocks * 4;       // 2 x Seg
+constexpr int kBmListBlocks = 96;                              // blocks of 32 rows a segment can finish, at most
+constexpr uint32_t kBmList = kBmRaw + 2 * 16384;               // 2 x finished blocks of a segment
+constexpr uint32_t kBmSeg = kBmList + 2 * kBmListBlocks * 4;   // 2 x Seg
 constexpr uint32_t kBmSegSlot = 192;
-constexpr uint32_t kBmMbarDesc = kBmSeg + 2 * kBmSegSlot;
+constexpr uint32_t kBmDone = kBmSeg + 2 * kBmSegSlot;          // 2 x Seg: the segments the lists belong to
+constexpr uint32_t kBmMbarDesc = kBmDone + 2 * kBmSegSlot;
 constexpr uint32_t kBmMbarX = kBmMbarDesc + 16;
 constexpr uint32_t kBmMbarB = kBmMbarX + 16;
-constexpr uint32_t kBmNext = kBmMbarB + 16;                    // 2 ints: next duo of the segment in a slot
-constexpr uint32_t kBmFlag = kBmNext + 8;
-constexpr uint32_t kBmCount = kBmFlag + 4;                     // finished blocks in the list (last segment)
-constexpr uint32_t kBmSmem = kBmCount + 4 + 1024;              // + slack for the alignment
+constexpr uint32_t kBmMbarL = kBmMbarB + 16;                   // a segment's list is complete
+constexpr uint32_t kBmNext = kBmMbarL + 16;                    // 2 ints: next duo of the segment in a slot
+constexpr uint32_t kBmCount = kBmNext + 8;                     // 2 ints: finished blocks in a list
+constexpr uint32_t kBmFlag = kBmCount + 8;
+constexpr uint32_t kBmSmem = kBmFlag + 8 + 1024;               // + slack for the alignment
 static_assert(sizeof(Seg) <= kBmSegSlot, "Seg must fit its slot");
-static_assert(kChunkDuos / 2 + 1 <= kBmListBlocks, "a segment's blocks are one round of counter updates");
-static_assert(kBmBBytes % 16 == 0 && kBmRaw % 16 == 0 && kBmStage % 16 == 0, "bulk copies and cp.async want 16-byte alignment");
+static_assert(kChunkDuos / 2 + 1 <= kBmListBlocks, "a segment's blocks fit a list");
+static_assert(kBmBBytes % 16 == 0 && kBmRaw % 16 == 0 && kBmList % 16 == 0 && kBmSeg % 16 == 0, "bulk copies want 16-byte alignment");
 
 __device__ __forceinline__ uint2 lds_v2(uint32_t addr) {
     uint2 v;
@@ -215,13 +217,41 @@ __global__ void __launch_bounds__(256) build_codes_kernel(const uint8_t *__restr
     }
 }
 
+// The listed blocks of a segment: outputs from their accumulators, which are cleared (with the block's
+// counter) for the next launch; `warps` warps take them in turn, straight from L2, a lane a row.  A
+// function of its own, so that the streaming loop keeps its registers.
+template <int MT>
+__device__ __noinline__ void finish_blocks(const Seg &sg, const int *list, int count, int m, int warp, int warps, int lane) {
+    for (int e = warp; e < count; e += warps) {
+        const int blk = list[e];
+        const float4 *sp = (const float4 *)sg.acc + (long long)(blk * kBlockRows + lane) * (MT / 4);
+        float v[MT];
+#pragma unroll
+        for (int qd = 0; qd < MT / 4; ++qd) {
+            const float4 f = __ldcg(sp + qd);
+            v[4 * qd] = f.x; v[4 * qd + 1] = f.y; v[4 * qd + 2] = f.z; v[4 * qd + 3] = f.w;
+        }
+        const int row = blk * kBlockRows + lane;
+        __syncwarp();            // every lane has read its row before any of it is cleared
+        float4 *ap = (float4 *)sg.acc + (long long)blk * (kBlockRows * MT / 4);
+#pragma unroll
+        for (int c = 0; c < kBlockRows * MT / 128; ++c) ap[c * 32 + lane] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (row < sg.n) {
+            const float bias = sg.bias ? __half2float(__ushort_as_half(sg.bias[row])) : 0.f;
+#pragma unroll
+            for (int rr = 0; rr < MT; ++rr)
+                if (rr < m) store_y(sg.y, (long long)rr * sg.n + row, v[rr] + bias, sg.y_dtype);
+        }
+        if (lane == 0) sg.counters[blk] = 0;
+    }
+}
+
 template <int Q, int GPW, int NT, bool CODES>
 __global__ void __launch_bounds__(kBmThreads, 1) batch_mma_kernel(const __grid_constant__ GemvArgs a) {
     static_assert(Q == 2 || Q == 3, "byte tables hold at most eight codes");
     extern __shared__ __align__(1024) unsigned char smem_dyn[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     constexpr int MT = 8 * NT;                     // rows of x the accumulators hold
-    constexpr int kBlockBytes = kBlockRows * MT * 4;
     const int m = a.batch_rows;
 
     const uint32_t sraw = smem_u32(smem_dyn);
@@ -235,7 +265,8 @@ __global__ void __launch_bounds__(kBmThreads, 1) batch_mma_kernel(const __grid_c
     const int spin = a.spin_limit;
     Seg *ring = (Seg *)(sm + kBmSeg);
     int *next_duo = (int *)(sm + kBmNext);
-    const uint32_t mb_desc = sbase + kBmMbarDesc, mb_x = sbase + kBmMbarX, mb_b = sbase + kBmMbarB;
+    const uint32_t mb_desc = sbase + kBmMbarDesc, mb_x = sbase + kBmMbarX, mb_b = sbase + kBmMbarB,
+                   mb_l = sbase + kBmMbarL;
 
     pdl_launch_dependents();
     if (tid == 0) {
@@ -243,6 +274,7 @@ __global__ void __launch_bounds__(kBmThreads, 1) batch_mma_kernel(const __grid_c
             mbar_init(mb_desc + 8 * i, 1);
             mbar_init(mb_x + 8 * i, 1);
             mbar_init(mb_b + 8 * i, 1);
+            mbar_init(mb_l + 8 * i, 1);
         }
         mbar_init_fence();
         *fail = 0;
@@ -272,38 +304,10 @@ __global__ void __launch_bounds__(kBmThreads, 1) batch_mma_kernel(const __grid_c
             *(uint2 *)(dst + row * kBmRowStride + qtr * kBmQuarterStride + (un & 31) * 8) = make_uint2(lo, hi);
         }
     };
-    // One finished block of 32 rows by one warp: outputs from its accumulators, which are cleared (with
-    // the block's counter) for the next launch.  v: the lane's row of the block.
-    auto write_block = [&](const Seg &sg, int blk, const float (&v)[MT]) {
-        const int row = blk * kBlockRows + lane;
-        float4 *ap = (float4 *)((unsigned char *)sg.acc + (long long)blk * kBlockBytes);
-#pragma unroll
-        for (int c = 0; c < kBlockBytes / 512; ++c) ap[c * 32 + lane] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (row < sg.n) {
-            const float bias = sg.bias ? __half2float(__ushort_as_half(sg.bias[row])) : 0.f;
-#pragma unroll
-            for (int rr = 0; rr < MT; ++rr)
-                if (rr < m) store_y(sg.y, (long long)rr * sg.n + row, v[rr] + bias, sg.y_dtype);
-        }
-        if (lane == 0) sg.counters[blk] = 0;
-    };
-    // The last segment of a CTA: nothing is left to stream, so all its warps take the finished blocks of
-    // the list in turn, straight from L2.
-    auto finish_list = [&](const Seg &sg) {
-        const int *list = (const int *)(sm + kBmList);
-        const int nlist = *(const int *)(sm + kBmCount);
-        for (int e = warp; e < nlist; e += kBmWarps + 1) {
-            const int blk = list[e];
-            const float4 *sp = (const float4 *)((const unsigned char *)sg.acc + (long long)blk * kBlockBytes) + lane * (MT / 4);
-            float v[MT];
-#pragma unroll
-            for (int qd = 0; qd < MT / 4; ++qd) {
-                const float4 f = __ldcg(sp + qd);
-                v[4 * qd] = f.x; v[4 * qd + 1] = f.y; v[4 * qd + 2] = f.z; v[4 * qd + 3] = f.w;
-            }
-            __syncwarp();        // every lane has read its row before any of it is cleared
-            write_block(sg, blk, v);
-        }
+    // the blocks that the segment in `slot` finished, as the control warp listed them
+    auto finish_segment = [&](int slot, int warps) {
+        finish_blocks<MT>(*(const Seg *)(sm + kBmDone + slot * kBmSegSlot), (const int *)(sm + kBmList) + slot * kBmListBlocks,
+                          ((const int *)(sm + kBmCount))[slot], m, warp, warps, lane);
     };
 
     if (warp == kBmWarps) {
@@ -359,73 +363,54 @@ __global__ void __launch_bounds__(kBmThreads, 1) batch_mma_kernel(const __grid_c
             if (l1) arrange(1, 1, ring[1].x_dtype);
         }
         pdl_wait();       // before this warp's first global write
-        int *list = (int *)(sm + kBmList);
         for (int i = 0;; ++i) {
             const int slot = i & 1;
             const bool have = mbar_wait_bounded(mb_desc + 8 * slot, (i >> 1) & 1, fail, spin);
             const Seg sg = ring[slot];
             if (!have || !sg.live) break;
             named_bar_sync_dyn(kBmBarSegDone + slot, kBmThreads);      // the consumers are done with it
-            // the last segment keeps its descriptor: the consumers finish its blocks with this warp
+            // for the list of its finished blocks (the slot's next descriptor overwrites the ring's copy)
+            for (int e = lane; e < (int)(sizeof(Seg) / 4); e += 32)
+                ((uint32_t *)(sm + kBmDone + slot * kBmSegSlot))[e] = ((const uint32_t *)&ring[slot])[e];
+            __syncwarp();
             const bool last = !ring[slot ^ 1].live;
             const bool live2 = last ? false : emit(slot);              // segment i + 2
             // its activations first, then publish: count finished duos per block of 32 rows; the
-            // blocks this segment completes are collected (128 candidates at a time), then turned
-            // into outputs (and cleared, with their counters, for the next launch) through a
-            // staging area, 16 blocks per round trip
+            // blocks this segment completes are listed for the consumers, who turn them into outputs
+            // when they are through with the next segment (or right away if this was the last)
             if (live2) arrange(slot, i + 2, ring[slot].x_dtype);
+            int *list = (int *)(sm + kBmList) + slot * kBmListBlocks;
             const int bfirst = sg.duo_a >> 1, blast = (sg.duo_b - 1) >> 1;
             const unsigned total = (unsigned)sg.slices * 2u;
             __threadfence();
-            for (int b0 = bfirst; b0 <= blast; b0 += kBmListBlocks) {
-                int nlist = 0;
-                bool mine[kBmListBlocks / 32];
+            int nlist = 0;
+            bool mine[kBmListBlocks / 32];
 #pragma unroll
-                for (int e = 0; e < kBmListBlocks / 32; ++e) {
-                    const int bi = b0 + 32 * e + lane;
-                    mine[e] = false;
-                    if (bi <= blast) {
-                        const int lo = max(sg.duo_a, 2 * bi), hi = min(sg.duo_b, 2 * bi + 2);
-                        const unsigned cnt = (unsigned)(hi - lo);
-                        mine[e] = atomicAdd(&sg.counters[bi], cnt) + cnt == total;
-                    }
+            for (int e = 0; e < kBmListBlocks / 32; ++e) {
+                const int bi = bfirst + 32 * e + lane;
+                mine[e] = false;
+                if (bi <= blast) {
+                    const int lo = max(sg.duo_a, 2 * bi), hi = min(sg.duo_b, 2 * bi + 2);
+                    const unsigned cnt = (unsigned)(hi - lo);
+                    mine[e] = atomicAdd(&sg.counters[bi], cnt) + cnt == total;
                 }
+            }
 #pragma unroll
-                for (int e = 0; e < kBmListBlocks / 32; ++e) {
-                    const unsigned mask = __ballot_sync(0xffffffffu, mine[e]);
-                    if (mine[e]) list[nlist + __popc(mask & ((1u << lane) - 1u))] = b0 + 32 * e + lane;
-                    nlist += __popc(mask);
-                }
-                __syncwarp();
-                if (nlist) __threadfence();
-                if (last) {
-                    if (lane == 0) *(int *)(sm + kBmCount) = nlist;
-                    named_bar_sync<kBmBarAll, kBmThreads>();
-                    finish_list(sg);
-                    break;
-                }
-                for (int l0 = 0; l0 < nlist; l0 += kBmStageBlocks) {
-                    const int nb = min(kBmStageBlocks, nlist - l0);
-                    for (int e = 0; e < nb; ++e) {
-                        const unsigned char *src = (const unsigned char *)sg.acc + (long long)list[l0 + e] * kBlockBytes;
-#pragma unroll
-                        for (int c = 0; c < kBlockBytes / 512; ++c)
-                            cp_async_16(sbase + kBmStage + e * kBlockBytes + (c * 32 + lane) * 16, src + (c * 32 + lane) * 16);
-                    }
-                    cp_async_wait_all();
-                    __syncwarp();
-                    for (int e = 0; e < nb; ++e) {
-                        const float4 *sp = (const float4 *)(sm + kBmStage + e * kBlockBytes + lane * (MT * 4));
-                        float v[MT];
-#pragma unroll
-                        for (int qd = 0; qd < MT / 4; ++qd) {
-                            const float4 f = sp[qd];
-                            v[4 * qd] = f.x; v[4 * qd + 1] = f.y; v[4 * qd + 2] = f.z; v[4 * qd + 3] = f.w;
-                        }
-                        write_block(sg, list[l0 + e], v);
-                    }
-                    __syncwarp();
-                }
+            for (int e = 0; e < kBmListBlocks / 32; ++e) {
+                const unsigned mask = __ballot_sync(0xffffffffu, mine[e]);
+                if (mine[e]) list[nlist + __popc(mask & ((1u << lane) - 1u))] = bfirst + 32 * e + lane;
+                nlist += __popc(mask);
+            }
+            if (nlist) __threadfence();
+            __syncwarp();
+            if (lane == 0) {
+                ((int *)(sm + kBmCount))[slot] = nlist;
+                if (!last) mbar_arrive(mb_l + 8 * slot);
+            }
+            if (last) {                  // nothing is left to stream: this warp helps
+                named_bar_sync<kBmBarAll, kBmThreads>();
+                finish_segment(slot, kBmWarps + 1);
+                break;
             }
         }
         if (*fail && lane == 0) atomicExch(a.status, 1);
@@ -519,12 +504,14 @@ __global__ void __launch_bounds__(kBmThreads, 1) batch_mma_kernel(const __grid_c
         // hand this segment to the control warp, then the first loads of the next one (an
         // arrival waits for the loads its thread has in flight)
         const bool have = mbar_wait_bounded(mb_desc + 8 * (slot ^ 1), ((i + 1) >> 1) & 1, fail, spin);
+        // what the segment before finished: listed by now, while this one was streamed
+        if (i && mbar_wait_bounded(mb_l + 8 * (slot ^ 1), ((i - 1) >> 1) & 1, fail, spin)) finish_segment(slot ^ 1, kBmWarps);
         named_bar_arrive_dyn(kBmBarSegDone + slot, kBmThreads);
         const Seg &nx = ring[slot ^ 1];
         if (!have) break;
         if (!nx.live) {
             named_bar_sync<kBmBarAll, kBmThreads>();
-            finish_list(ring[slot]);
+            finish_segment(slot, kBmWarps + 1);
             break;
         }
         open_segment(nx);
