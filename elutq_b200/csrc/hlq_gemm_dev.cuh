@@ -32,6 +32,9 @@ struct GemmArgs {
     int y_dtype;
 };
 
+// programmatic dependent launch: the next kernel of the stream may start / everything before has finished
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
     return (uint32_t)__cvta_generic_to_shared(p);
 }
@@ -215,8 +218,6 @@ inline EncodeTiledFn encode_fn() {
 // two slabs: K is not split).
 int launch_dequant_gemm_pair(const GemmArgs &a, int q, const void *x, int sms, float *acc, size_t acc_bytes,
                              cudaStream_t stream);
-// tokens per pair tile and (optionally) waves x tokens as a cost to compare tilings by
-int pair_tile_tokens(int n, int m, int sms, double *cost);
 
 }  // namespace gemm
 }  // namespace hlq

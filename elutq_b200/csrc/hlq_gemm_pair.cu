@@ -38,10 +38,17 @@
 // thread whose waits and commits left the pipe idle (now two, alternating), tiles launched as
 // CTAs (now persistent).
 //
+// Launched with programmatic dependent launch, as are the conversion of bf16 tokens and the finishing
+// kernel: barriers, tables, tensor memory and a pair's first weights (5 us of the 12.5 that a 4096x4096
+// product of 48 tokens takes) are ready when the kernel before ends.  Seven projections of a Llama-3-8B
+// layer, 3 bits, 48 tokens, call by call: 174 -> 135 us.
+//
 // Precision and operand formats as in hlq_gemm.cu.  All waits are bounded (poll limit); the first
 // that runs out sets the CTA's failure flag, later waits give up at once, both CTAs still meet at
 // the cluster barriers and tensor memory is always released.
 #include <cuda.h>
+
+#include <algorithm>
 
 #include "hlq_gemm_dev.cuh"
 
@@ -50,7 +57,7 @@ namespace gemm {
 
 namespace {
 
-constexpr uint32_t kByteTableBytes = 4096;                      // byte tables of two- and three-plane weights
+constexpr uint32_t kByteTableBytes = 4096;                      // byte tables of weights of two to four planes
 constexpr int kPairStepK = 128;                                  // channels per K step: a quarter of a slice
 constexpr int kPairStages = 4;                                   // K steps in flight (both operands): one slice
 constexpr int kPairDeqWarps = 16;
@@ -118,7 +125,7 @@ __device__ __forceinline__ void umma_commit_pair(uint32_t cluster_mbar) {
                  : "memory");
 }
 
-// ---- two- and three-plane weights: a byte of a plane (8 channels) is looked up whole --------------
+// ---- weights of two to four planes: a byte of a plane (8 channels) is looked up whole --------------
 // Two planes: entry b of table p is, for the 8 channels of plane byte b, one selector byte per
 // channel (.x channels 0..3, .y channels 4..7): 0x10 + 0x22 bit for plane 0, 0x44 bit for plane 1;
 // the OR of the two entries selects, per pair of channels, the fp16 values z + b0 a0 + b1 a1 out of
@@ -127,6 +134,8 @@ __device__ __forceinline__ void umma_commit_pair(uint32_t cluster_mbar) {
 // three entries is the 3-bit code of 8 channels, which indexes byte tables of the 8 possible values
 // (their low bytes in two registers, their high bytes in two): two prmt gather 4 low and 4 high
 // bytes, two more pair them up.
+// Four planes: the same with 16 values, each byte table in two halves; the code's top bit, spread to a byte
+// mask by one prmt, picks between the two lookups.  4096x4096, 17 tokens: 20.1 us with nibble masks, 18.2 so.
 // Either way a weight costs about half the ALU instructions of the nibble-mask form and the 2^q
 // values of a group are rounded to fp16 once, from fp32.
 template <int Q>
@@ -143,9 +152,9 @@ __device__ __forceinline__ void fill_byte_tables(int tid, int nthreads, unsigned
             }
             t[e] = make_uint2(lo, hi);
         }
-    } else if constexpr (Q == 3) {
+    } else if constexpr (Q == 3 || Q == 4) {
         uint32_t *t = (uint32_t *)tab;                 // [plane][256]
-        for (int e = tid; e < 768; e += nthreads) {
+        for (int e = tid; e < 256 * Q; e += nthreads) {
             const int p = e >> 8, b = e & 255;
             uint32_t w = 0u;
             for (int c = 0; c < 8; ++c)
@@ -162,7 +171,7 @@ __device__ __forceinline__ uint32_t prmt_b32(uint32_t a, uint32_t b, uint32_t se
 // the values a weight of one group can take, as prmt sources
 template <int Q>
 struct GroupValues {
-    uint32_t v[Q == 2 ? 2 : 4];      // q = 2: {v0, v1}, {v2, v3} as fp16 pairs; q = 3: low bytes x2, high bytes x2
+    uint32_t v[1 << (Q - 1)];      // q = 2: {v0, v1}, {v2, v3} as fp16 pairs; else: low bytes of four values each, then high bytes
 };
 template <int Q>
 __device__ __forceinline__ void group_values(GroupValues<Q> &gv, const uint16_t (&alpha)[Q], uint16_t zero) {
@@ -181,10 +190,12 @@ __device__ __forceinline__ void group_values(GroupValues<Q> &gv, const uint16_t 
         gv.v[0] = pr[0];
         gv.v[1] = pr[1];
     } else {
-        gv.v[0] = prmt_b32(pr[0], pr[1], 0x6420u);     // low bytes of values 0..3
-        gv.v[1] = prmt_b32(pr[2], pr[3], 0x6420u);     // 4..7
-        gv.v[2] = prmt_b32(pr[0], pr[1], 0x7531u);     // high bytes of values 0..3
-        gv.v[3] = prmt_b32(pr[2], pr[3], 0x7531u);     // 4..7
+        constexpr int H = (1 << Q) / 4;
+#pragma unroll
+        for (int e = 0; e < H; ++e) {
+            gv.v[e] = prmt_b32(pr[2 * e], pr[2 * e + 1], 0x6420u);         // low bytes of values 4 e .. 4 e + 3
+            gv.v[H + e] = prmt_b32(pr[2 * e], pr[2 * e + 1], 0x7531u);     // their high bytes
+        }
     }
 }
 // 32 channels (bits[p] = the 32 bits of plane p in channel order) as 16 fp16 pairs
@@ -206,12 +217,21 @@ __device__ __forceinline__ void expand32(const uint32_t (&bits)[Q], const GroupV
         const uint32_t *t = (const uint32_t *)tab;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            const uint32_t code = t[(bits[0] >> (8 * k)) & 0xffu] | t[256 + ((bits[1] >> (8 * k)) & 0xffu)] |
-                                  t[512 + ((bits[2] >> (8 * k)) & 0xffu)];
+            uint32_t code = t[(bits[0] >> (8 * k)) & 0xffu] | t[256 + ((bits[1] >> (8 * k)) & 0xffu)] |
+                            t[512 + ((bits[2] >> (8 * k)) & 0xffu)];
+            if constexpr (Q == 4) code |= t[768 + ((bits[Q - 1] >> (8 * k)) & 0xffu)];
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const uint32_t sel = h ? code >> 16 : code;
-                const uint32_t lb = prmt_b32(gv.v[0], gv.v[1], sel), hb = prmt_b32(gv.v[2], gv.v[3], sel);
+                uint32_t lb, hb;
+                if constexpr (Q == 3) {
+                    lb = prmt_b32(gv.v[0], gv.v[1], sel);
+                    hb = prmt_b32(gv.v[2], gv.v[3], sel);
+                } else {
+                    const uint32_t s3 = sel & 0x7777u, upper = prmt_b32(sel << 4, sel, 0xd9c8u);   // bit 3 of nibble i as byte i
+                    lb = (prmt_b32(gv.v[0], gv.v[1], s3) & ~upper) | (prmt_b32(gv.v[2], gv.v[3], s3) & upper);
+                    hb = (prmt_b32(gv.v[4], gv.v[5], s3) & ~upper) | (prmt_b32(gv.v[6], gv.v[7], s3) & upper);
+                }
                 o[4 * k + 2 * h] = prmt_b32(lb, hb, 0x5140u);
                 o[4 * k + 2 * h + 1] = prmt_b32(lb, hb, 0x7362u);
             }
@@ -312,6 +332,9 @@ dequant_gemm_pair_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap x
         return grp * a.tok_group + rem % width;
     };
 
+    // The next kernel of the stream may set itself up (barriers, tables, tensor memory, its first weights)
+    // on SMs this one leaves; tokens are read and outputs written only after the kernel before has ended.
+    pdl_launch_dependents();
     if (tid == 0) {
         for (int s = 0; s < kPairStages; ++s) {
             mbar_init(bar_full + 8 * s, 1 + 2 * 4);             // producer of CTA 0; the four warps of the step, both CTAs
@@ -325,7 +348,7 @@ dequant_gemm_pair_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap x
         *fail = 0;
     }
     if (tid < 16) fill_dequant_tables(tid, lut, sel_lut);
-    if constexpr (Q == 2 || Q == 3) fill_byte_tables<Q>(tid, kPairThreads, tiles_ptr + kPairStages * kPairXStage + 256);
+    if constexpr (Q >= 2) fill_byte_tables<Q>(tid, kPairThreads, tiles_ptr + kPairStages * kPairXStage + 256);
     if (warp == 1) {   // all of tensor memory, in both CTAs with one instruction each
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
                      "r"(kPairTmemCols) : "memory");
@@ -350,6 +373,7 @@ dequant_gemm_pair_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap x
             const uint32_t xbytes = (uint32_t)a.tile_m * kPairStepK * 2;  // both halves, both boxes
             int g = 0;
             bool ok = true;
+            pdl_wait();
             for (int u = pair; u < nunits && ok; u += npairs) {
                 const int m0 = tok_tile_of(unit_tile(u)) * a.tile_m;
                 for (int kt = 4 * unit_s0(u); kt < 4 * unit_s1(u); ++kt, ++g) {
@@ -424,6 +448,7 @@ dequant_gemm_pair_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap x
             const int row = row_tile_of(tile) * 256 + 128 * (int)rank + t;
             const int m0 = tok_tile_of(tile) * a.tile_m;
             pair_wait(bar_acc, parity, fail);
+            pdl_wait();                              // before this warp's first global write
             tc_fence_after();
             float bv = 0.f;
             if (a.bias && row < a.n) bv = __half2float(__ushort_as_half(a.bias[row]));
@@ -533,7 +558,7 @@ dequant_gemm_pair_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap x
                 // weights are made before the wait for the stage (it is busy for as long as the products
                 // that read it, and the arithmetic need not wait for them), the other half after.
                 const int s = part;
-                GroupValues<(Q == 2 || Q == 3) ? Q : 2> gv;
+                GroupValues<Q >= 2 ? Q : 2> gv;
                 auto make = [&](int ws, uint32_t (&o)[16]) {                  // 32 channels of the lane's 128
                     const int u = ((ws * a.gpw) >> 2) ^ gsel;
                     uint32_t bits[Q];
@@ -543,13 +568,13 @@ dequant_gemm_pair_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap x
                     // per slice, g = 64: twice, g = 32: for every 32 channels)
                     const bool fresh = ws == 0 || a.gpw == 4 || (a.gpw == 2 && ws == 2);
                     uint16_t al[Q], z = 0;
-                    if (fresh || !(Q == 2 || Q == 3)) {
+                    if (fresh || Q < 2) {
 #pragma unroll
                         for (int p = 0; p < Q; ++p)
                             al[p] = (uint16_t)((((uint64_t)cur.mt[p].y << 32 | cur.mt[p].x) >> (16 * u)) & 0xffffu);
                         z = (uint16_t)((((uint64_t)cur.mt[Q].y << 32 | cur.mt[Q].x) >> (16 * u)) & 0xffffu);
                     }
-                    if constexpr (Q == 2 || Q == 3) {
+                    if constexpr (Q >= 2) {
                         if (fresh) group_values<Q>(gv, al, z);
                         expand32<Q>(bits, gv, byte_tab, o);
                     } else {
@@ -611,39 +636,73 @@ dequant_gemm_pair_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap x
 
 // Finishes a launch whose K was split: y = sum of the parts' slabs (+ bias) in the output type.
 // The parts are added in their order, so the result is the same in every run.
-__global__ void pair_finish_kernel(const float *__restrict__ acc, void *__restrict__ y, const uint16_t *__restrict__ bias,
-                                   long long total, int n, int parts, int y_dtype) {
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-        float o = 0.f;
-        for (int p = 0; p < parts; ++p) o += __ldcs(acc + (long long)p * total + i);
-        if (bias) o += __half2float(__ushort_as_half(bias[i % n]));
-        if (y_dtype == HLQ_F16) ((__half *)y)[i] = __float2half_rn(o);
-        else if (y_dtype == HLQ_BF16) ((__nv_bfloat16 *)y)[i] = __float2bfloat16_rn(o);
-        else ((float *)y)[i] = o;
+// VEC: four outputs a thread (n a multiple of four), else one.
+template <bool VEC>
+__global__ void __launch_bounds__(256) pair_finish_kernel(const float *__restrict__ acc, void *__restrict__ y,
+                                                          const uint16_t *__restrict__ bias, long long total, int n, int parts,
+                                                          int y_dtype) {
+    constexpr int W = VEC ? 4 : 1;
+    pdl_launch_dependents();
+    pdl_wait();
+    const long long stride = (long long)gridDim.x * blockDim.x * W;
+    for (long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * W; i < total; i += stride) {
+        float o[W] = {};
+#pragma unroll 4
+        for (int p = 0; p < parts; ++p) {
+            const float *src = acc + (long long)p * total + i;
+            if constexpr (VEC) {
+                const float4 v = __ldcs((const float4 *)src);
+                o[0] += v.x; o[1] += v.y; o[2] += v.z; o[3] += v.w;
+            } else {
+                o[0] += __ldcs(src);
+            }
+        }
+        if (bias) {
+            const int col = (int)(i % n);
+#pragma unroll
+            for (int e = 0; e < W; ++e) o[e] += __half2float(__ushort_as_half(bias[col + e]));
+        }
+#pragma unroll
+        for (int e = 0; e < W; ++e) {
+            if (y_dtype == HLQ_F16) ((__half *)y)[i + e] = __float2half_rn(o[e]);
+            else if (y_dtype == HLQ_BF16) ((__nv_bfloat16 *)y)[i + e] = __float2bfloat16_rn(o[e]);
+            else ((float *)y)[i + e] = o[e];
+        }
     }
 }
 
-// How many parts to split K into, by a cost in microseconds fitted to measurements on a B200: a
-// slice of 512 channels takes a pair about 1.8, a unit's first operands and its read-back 8, the
-// finishing kernel 4 plus its reads at 4 bytes per part and output.  At most max_parts slabs fit.
-int choose_ksplit(int ntiles, int slices, int pairs, long long outputs, int max_parts) {
-    int best_s = 1;
+// Tokens per tile (a multiple of 32 up to 256) and parts of K, chosen together by a cost in microseconds
+// fitted to measurements on a B200 (2 and 3 bits, 48 to 2048 tokens): a unit's first operands and its
+// read-back take 6.4 to 8.3, a slice of 512 channels 2.2 however narrow the tile is (the weights are made and the
+// products issued at that rate) and from 212 tokens on in proportion to the tile (the products themselves);
+// a split adds the finishing kernel, 2.7, and 1.4 per million fp32 sums written and read.  At most max_parts
+// slabs fit; K is split only where there are fewer tiles than pairs.  Against a tile chosen by waves alone
+// and a split chosen after it: 4096x14336, 256 / 512 tokens 47.8 -> 33.7 / 77.7 -> 53.5 us; 4096x4096,
+// 333 / 512 tokens 27.0 -> 23.7 / 28.9 -> 26.2; 1000x1536, 48 tokens 11.0 -> 8.0.
+void choose_plan(int n, int m, int slices, int pairs, int max_parts, int *tile_m, int *ksplit) {
     double best = -1.0;
-    for (int sp = 1; sp <= slices && sp <= max_parts && sp <= 16; ++sp) {
-        const long long rounds = ((long long)ntiles * sp + pairs - 1) / pairs;
-        const double unit = 1.8 * ((slices + sp - 1) / sp) + 8.0;
-        const double cost = rounds * unit + (sp > 1 ? 4.0 + 4.0e-6 * sp * outputs / 4.0 : 0.0);
-        if (best < 0 || cost < best * 0.97) {      // a split must win clearly
-            best = cost;
-            best_s = sp;
+    const long long row_tiles = (n + 255) / 256;
+    const int fewest = (m + 255) / 256;
+    for (int tt = fewest; tt <= 2 * fewest + 2; ++tt) {       // the tokens in tt tiles, all of one width
+        const int tm = ((m + tt - 1) / tt + 31) / 32 * 32;
+        const long long tiles = row_tiles * ((m + tm - 1) / tm);
+        const double unit = 6.4 + 0.0075 * tm, per_slice = tm > 212 ? 2.2 * tm / 212 : 2.2;
+        for (int sp = 1; sp <= slices && sp <= max_parts && sp <= 16; ++sp) {
+            if (sp > 1 && tiles >= pairs) break;
+            const long long rounds = (tiles * sp + pairs - 1) / pairs;
+            const double cost = rounds * (unit + per_slice * ((slices + sp - 1) / sp)) +
+                                (sp > 1 ? 2.7 + 1.4e-6 * sp * (double)m * n : 0.0);
+            if (best < 0 || cost < best * 0.98) {      // a narrower tile or a further split must win clearly
+                best = cost;
+                *tile_m = tm;
+                *ksplit = sp;
+            }
         }
     }
-    return best_s;
 }
 
 template <int Q>
-int launch_pair_inst(GemmArgs &a, const CUtensorMap &xmap, int ntiles, size_t acc_bytes, cudaStream_t stream) {
+int launch_pair_inst(GemmArgs &a, const void *x, EncodeTiledFn enc, size_t acc_bytes, cudaStream_t stream) {
     static int pairs_cached[64] = {};        // clusters of two that run at once, per device; 0 = not asked yet
     int dev = 0;
     HLQ_CUDA(cudaGetDevice(&dev));
@@ -667,58 +726,14 @@ int launch_pair_inst(GemmArgs &a, const CUtensorMap &xmap, int ntiles, size_t ac
         if (nclusters < 1) return HLQ_ERR_UNSUPPORTED;
         pairs = nclusters;
     }
-    // few tiles: split K, if the workspace has room for the fp32 sums
-    a.ksplit = 1;
     const long long total = (long long)a.m * a.n;
-    if (ntiles < pairs && a.acc && acc_bytes >= 2 * (size_t)total * sizeof(float))
-        a.ksplit = choose_ksplit(ntiles, a.kp / 512, pairs, total, (int)(acc_bytes / ((size_t)total * sizeof(float))));
-    const int nunits = ntiles * a.ksplit;
-    const int use = nunits < pairs ? nunits : pairs;
-    kernel<<<2 * use, kPairThreads, kPairDynSmem, stream>>>(a, xmap);
-    count_launch();
-    int rc = note_cuda(cudaGetLastError());
-    if (rc || a.ksplit == 1) return rc;
-    long long blocks = (total + 255) / 256;
-    if (blocks > 148 * 8) blocks = 148 * 8;
-    pair_finish_kernel<<<(int)blocks, 256, 0, stream>>>(a.acc, a.y, a.bias, total, a.n, a.ksplit, a.y_dtype);
-    count_launch();
-    return note_cuda(cudaGetLastError());
-}
-
-}  // namespace
-
-// Tokens per pair tile: a multiple of 32 from 128 to 256 that wastes the fewest waves of SM pairs.
-int pair_tile_tokens(int n, int m, int sms, double *cost) {
-    const int pairs = sms / 2 > 0 ? sms / 2 : 1;
-    double best = 1e300;
-    int tile = 256;
-    const int lo = m >= 128 ? 128 : ((m + 31) / 32 * 32);
-    for (int tm = 256; tm >= lo; tm -= 32) {
-        const long long tiles = (long long)((n + 255) / 256) * ((m + tm - 1) / tm);
-        const long long waves = (tiles + pairs - 1) / pairs;
-        const double c = (double)waves * tm;
-        if (c < best * 0.999) {
-            best = c;
-            tile = tm;
-        }
-    }
-    if (cost) *cost = best;
-    return tile;
-}
-
-int launch_dequant_gemm_pair(const GemmArgs &a_in, int q, const void *x, int sms, float *acc, size_t acc_bytes,
-                             cudaStream_t stream) {
-    if (a_in.m < 1 || sms < 2) return HLQ_ERR_UNSUPPORTED;
-    EncodeTiledFn enc = encode_fn();
-    if (!enc) return HLQ_ERR_NO_DEVICE;
-    GemmArgs a = a_in;
-    a.acc = acc;
-    a.tile_m = pair_tile_tokens(a.n, a.m, sms, nullptr);
+    const int max_parts = a.acc ? (int)std::min<size_t>(acc_bytes / ((size_t)total * sizeof(float)), 16) : 1;
+    choose_plan(a.n, a.m, a.kp / 512, pairs, max_parts > 1 ? max_parts : 1, &a.tile_m, &a.ksplit);
+    const int tok_tiles = (a.m + a.tile_m - 1) / a.tile_m;
     {
         // token tiles whose activations (tile_m x k fp16 each) fit a third of a B200's L2 together
         const long long tile_bytes = (long long)a.tile_m * a.k * 2, budget = 40ll << 20;
-        const int tok_tiles = (a.m + a.tile_m - 1) / a.tile_m;
-        long long g = budget / (tile_bytes > 0 ? tile_bytes : 1);
+        const long long g = budget / (tile_bytes > 0 ? tile_bytes : 1);
         a.tok_group = (int)(g < 1 ? 1 : (g > tok_tiles ? tok_tiles : g));
     }
     CUtensorMap xmap;
@@ -730,12 +745,32 @@ int launch_dequant_gemm_pair(const GemmArgs &a_in, int q, const void *x, int sms
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return HLQ_ERR_INVALID_ARGUMENT;
-    const int ntiles = ((a.n + 255) / 256) * ((a.m + a.tile_m - 1) / a.tile_m);
+    const int ntiles = ((a.n + 255) / 256) * tok_tiles;
+    const int nunits = ntiles * a.ksplit;
+    const int use = nunits < pairs ? nunits : pairs;
+    const int rc = launch_pdl(kernel, dim3(2 * use), dim3(kPairThreads), kPairDynSmem, stream, a, xmap);
+    if (rc || a.ksplit == 1) return rc;
+    const bool vec = a.n % 4 == 0 && ((uintptr_t)a.acc & 15) == 0;
+    long long blocks = (total / (vec ? 4 : 1) + 255) / 256;
+    if (blocks > 148 * 4) blocks = 148 * 4;
+    return launch_pdl(vec ? pair_finish_kernel<true> : pair_finish_kernel<false>, dim3((int)blocks), dim3(256), 0, stream,
+                      (const float *)a.acc, a.y, a.bias, total, a.n, a.ksplit, a.y_dtype);
+}
+
+}  // namespace
+
+int launch_dequant_gemm_pair(const GemmArgs &a_in, int q, const void *x, int sms, float *acc, size_t acc_bytes,
+                             cudaStream_t stream) {
+    if (a_in.m < 1 || sms < 2) return HLQ_ERR_UNSUPPORTED;
+    EncodeTiledFn enc = encode_fn();
+    if (!enc) return HLQ_ERR_NO_DEVICE;
+    GemmArgs a = a_in;
+    a.acc = acc;
     switch (q) {
-        case 1: return launch_pair_inst<1>(a, xmap, ntiles, acc_bytes, stream);
-        case 2: return launch_pair_inst<2>(a, xmap, ntiles, acc_bytes, stream);
-        case 3: return launch_pair_inst<3>(a, xmap, ntiles, acc_bytes, stream);
-        case 4: return launch_pair_inst<4>(a, xmap, ntiles, acc_bytes, stream);
+        case 1: return launch_pair_inst<1>(a, x, enc, acc_bytes, stream);
+        case 2: return launch_pair_inst<2>(a, x, enc, acc_bytes, stream);
+        case 3: return launch_pair_inst<3>(a, x, enc, acc_bytes, stream);
+        case 4: return launch_pair_inst<4>(a, x, enc, acc_bytes, stream);
     }
     return HLQ_ERR_SHAPE;
 }

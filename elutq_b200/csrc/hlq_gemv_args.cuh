@@ -235,24 +235,4 @@ extern std::mutex g_first_use;     // serializes the per-device lookups done on 
 // The device's SM count and shared-memory limit, looked up once; HLQ_ERR_NO_DEVICE unless sm_100.
 int device_info(int device, DeviceInfo **out);
 
-// Launch with programmatic stream serialization: the kernel may start while its predecessor
-// drains and orders itself with griddepcontrol.wait.
-template <typename KernelT, typename ArgsT>
-static int launch_pdl(KernelT kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                      const ArgsT &args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    HLQ_CUDA(cudaLaunchKernelEx(&cfg, kernel, args));
-    count_launch();
-    return HLQ_OK;
-}
-
 }  // namespace hlq

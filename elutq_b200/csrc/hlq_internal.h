@@ -80,6 +80,26 @@ void count_launch(int n = 1);
         if (e__ != cudaSuccess) return hlq::note_cuda(e__); \
     } while (0)
 
+// Launch with programmatic stream serialization: the kernel may start while its predecessor
+// drains and orders itself with griddepcontrol.wait.
+template <typename KernelT, typename... ArgsT>
+static int launch_pdl(KernelT kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                      const ArgsT &...args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    HLQ_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
+    count_launch();
+    return HLQ_OK;
+}
+
 // Workspace layout: [0, 256) header (int status at 0), then counters, then accumulators.
 constexpr size_t kWsHeader = 256;
 constexpr int kLutMaxM = 16;  // rows of x one LUT-GEMV launch handles
