@@ -1,4 +1,4 @@
-// Small batches (3..16 rows of activations) over HLQ weights in the streaming layout, sm_100a:
+// Small batches (3..16 rows of activations, 2 to 4 bits) over HLQ weights in the streaming layout, sm_100a:
 // the weights are streamed ONCE per call, whatever the number of rows.
 //
 // Replaces, for small m, the reference's batched path
@@ -134,6 +134,65 @@ __device__ __forceinline__ void load_batch_tile(BatchTile<Q, GPW, CODES> &t, con
         }
     }
 }
+// Four planes: sixteen values would want four registers per byte table and a select per lookup, so every
+// plane gets products of its own instead: A = alpha_p where the plane's bit is set, z everywhere in a fifth.
+// (word >> t) & 0x00010001 times the bits of alpha_p IS the fp16 pair of channels t and t + 16, one
+// integer multiply that does not compete with the shift and the mask.  All operands are exact, so the result
+// is rounded once, at the output (the LUT kernel's two-row passes round their table entries to fp16: 2-norm
+// error against 64 bits 2.8e-4 to 3.7e-4, here 2.1e-4, that of the output type alone).  An infinite
+// activation makes its row NaN (0 x inf).  From three rows on; two are one pass of the LUT kernel
+// (4096x4096, g = 64: 2 rows 12.3 us there; 8 rows 46.4 us in four passes, 13.3 here; 14336x4096, 8 rows
+// 90.8 and 31.3; 16 rows 161.8 and 41.7).
+template <int GPW, int NT>
+__device__ __forceinline__ void mma_tile_planes(const BatchTile<4, GPW, false> &t, uint32_t bs, int r, uint32_t usel,
+                                                float (&acc)[4 / NT][NT][4]) {
+    constexpr int kChains = 4 / NT;
+    constexpr int kWordsPerGroup = 4 / GPW;
+    constexpr int gshift = GPW == 1 ? 3 : (GPW == 2 ? 2 : 1);
+    const bool far = r & 4;
+    uint32_t al[2][4], z2[2];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        if (c % kWordsPerGroup == 0) {
+            const int u = (c / kWordsPerGroup) ^ ((r >> gshift) & (GPW - 1));
+#pragma unroll
+            for (int ou = 0; ou < 2; ++ou) {
+#pragma unroll
+                for (int p = 0; p < 4; ++p) al[ou][p] = tile_meta_bits<GPW>(t.mt[p], ou, u);
+                z2[ou] = tile_meta_bits<GPW>(t.mt[4], ou, u) * 0x00010001u;
+            }
+        }
+        uint32_t w[2][4];            // word c of the planes in source order (see source_order)
+#pragma unroll
+        for (int ou = 0; ou < 2; ++ou)
+#pragma unroll
+            for (int p = 0; p < 4; ++p) {
+                const uint4 &v = t.w[ou][p];
+                const uint32_t q0 = (c < 2) == !far ? v.x : v.z, q1 = (c < 2) == !far ? v.y : v.w;
+                w[ou][p] = c & 1 ? prmt(q1, q0, usel) : prmt(q0, q1, usel);
+            }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {       // channels 2u, 2u + 16, 2u + 1, 2u + 17 of the word, in each quarter
+            uint2 b[NT];
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt) {
+                b[nt] = lds_v2(bs + (uint32_t)((c * 8 + u) * 8) + nt * 8 * kBmRowStride);
+                mma_16816(acc[u % kChains][nt], z2[0], z2[1], z2[0], z2[1], b[nt].x, b[nt].y);
+            }
+#pragma unroll
+            for (int p = 0; p < 4; ++p) {
+                uint32_t a[2][2];
+#pragma unroll
+                for (int ou = 0; ou < 2; ++ou)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) a[ou][e] = ((w[ou][p] >> (2 * u + e)) & 0x00010001u) * al[ou][p];
+#pragma unroll
+                for (int nt = 0; nt < NT; ++nt)
+                    mma_16816(acc[(u + p + 1) % kChains][nt], a[0][0], a[1][0], a[0][1], a[1][1], b[nt].x, b[nt].y);
+            }
+        }
+    }
+}
 // One duo (16 rows x the slice's 512 channels) times the rows of x in shared memory.
 // `bs`: this lane's base into the fragment-ordered activations (its row of x and quarter).
 template <int Q, int GPW, int NT, bool CODES>
@@ -248,7 +307,7 @@ __device__ __noinline__ void finish_blocks(const Seg &sg, const int *list, int c
 
 template <int Q, int GPW, int NT, bool CODES>
 __global__ void __launch_bounds__(kBmThreads, 1) batch_mma_kernel(const __grid_constant__ GemvArgs a) {
-    static_assert(Q == 2 || Q == 3, "byte tables hold at most eight codes");
+    static_assert(Q >= 2 && Q <= 4 && (Q < 4 || !CODES), "byte tables hold at most eight codes");
     extern __shared__ __align__(1024) unsigned char smem_dyn[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     constexpr int MT = 8 * NT;                     // rows of x the accumulators hold
@@ -282,7 +341,8 @@ __global__ void __launch_bounds__(kBmThreads, 1) batch_mma_kernel(const __grid_c
     __syncthreads();
 
     // The slice's activations, as they came, into the order the B fragments read them:
-    // unit (row of x, quarter, word c, s, h) = channels 128 quarter + 32 c + 4 (4 h + e) + s, e = 0..3.
+    // unit (row of x, quarter, word c, s, h) = channels 128 quarter + 32 c + 4 (4 h + e) + s, e = 0..3;
+    // four planes: unit (.., word c, u) = channels 32 c + 2 u + (0, 16, 1, 17).
     auto arrange_units = [&](int slot, int x_dtype, int first, int step) {
         const uint16_t *raw = (const uint16_t *)(sm + kBmRaw) + slot * (16 * kSliceK);
         unsigned char *dst = sm + kBmB + slot * kBmBBytes;
@@ -291,11 +351,11 @@ __global__ void __launch_bounds__(kBmThreads, 1) batch_mma_kernel(const __grid_c
             const int qtr = un >> 5, c = (un >> 3) & 3, s = (un >> 1) & 3, h = un & 1;
             uint32_t lo = 0u, hi = 0u;
             if (row < m) {
-                const uint16_t *src = raw + row * kSliceK + 128 * qtr + 32 * c + 16 * h + s;
+                const uint16_t *src = raw + row * kSliceK + 128 * qtr + 32 * c + (Q == 4 ? 2 * (un & 7) : 16 * h + s);
                 uint16_t e[4];
 #pragma unroll
                 for (int q2 = 0; q2 < 4; ++q2) {
-                    e[q2] = src[4 * q2];
+                    e[q2] = src[Q == 4 ? 16 * (q2 & 1) + (q2 >> 1) : 4 * q2];
                     if (x_dtype != HLQ_F16) e[q2] = __half_as_ushort(__float2half_rn(x_to_float(e[q2], x_dtype)));
                 }
                 lo = (uint32_t)e[0] | ((uint32_t)e[1] << 16);
@@ -455,7 +515,8 @@ __global__ void __launch_bounds__(kBmThreads, 1) batch_mma_kernel(const __grid_c
     }
     auto run_tile = [&](const BatchTile<Q, GPW, CODES> &t, int d, uint32_t bs) {
         float accs[4 / NT][NT][4] = {};
-        mma_tile<Q, GPW, NT, CODES>(t, bs, r, usel, accs);
+        if constexpr (Q == 4) mma_tile_planes<GPW, NT>(t, bs, r, usel, accs);
+        else mma_tile<Q, GPW, NT, CODES>(t, bs, r, usel, accs);
         float acc[NT][4];
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt)
@@ -492,6 +553,12 @@ __global__ void __launch_bounds__(kBmThreads, 1) batch_mma_kernel(const __grid_c
         // beyond each warp's first are taken from a counter, so no warp idles at the segment's end
         while (cur < dend) {
             int nxt = take(slot);
+            if constexpr (Q == 4) {          // a tile of four planes: no registers for a second one
+                run_tile(t0, cur, bs);
+                if (nxt < dend) load_duo(t0, nxt);
+                cur = nxt;
+                continue;
+            }
             if (nxt < dend) load_duo(t1, nxt);
             run_tile(t0, cur, bs);
             cur = nxt;
@@ -536,7 +603,7 @@ int launch_inst(const GemvArgs &args, int ctas, cudaStream_t stream) {
 
 // Two rows of x are cheaper as one pass of the LUT kernel with half2 table entries (0.65 of this
 // kernel's time on the Llama-3-8B projection set); from three rows on this kernel wins.
-bool batch_mma_supported(int q, int m) { return (q == 2 || q == 3) && m >= 3 && m <= kLutMaxM; }
+bool batch_mma_supported(int q, int m) { return q >= 2 && q <= 4 && m >= 3 && m <= kLutMaxM; }
 
 // All `m` rows of x of the launch in one pass.  The accumulators of a job are [np][8 or 16] fp32
 // (rows of x innermost), the counters those of its first row.
@@ -557,6 +624,10 @@ int launch_batch_mma(int q, int gpw, const GemvArgs &a_in, int ctas, int m, cuda
     }
     HLQ_CASE(2, 1) HLQ_CASE(2, 2) HLQ_CASE(2, 4)
     HLQ_CASE(3, 1) HLQ_CASE(3, 2) HLQ_CASE(3, 4)
+#undef HLQ_CASE
+#define HLQ_CASE(GV) \
+    if (q == 4 && gpw == GV) return m <= 8 ? launch_inst<4, GV, 1, false>(a, ctas, stream) : launch_inst<4, GV, 2, false>(a, ctas, stream);
+    HLQ_CASE(1) HLQ_CASE(2) HLQ_CASE(4)
 #undef HLQ_CASE
     return HLQ_ERR_SHAPE;
 }

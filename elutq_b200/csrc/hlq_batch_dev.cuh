@@ -38,9 +38,9 @@ __device__ __forceinline__ void source_order(const uint4 &w, bool far, uint32_t 
     out[3] = prmt(q3, q2, usel);
 }
 
-// fp16 scale or zero of (plane-or-zero pp, oct ou, positional sub-group u) of a tile
+// fp16 scale or zero of (plane-or-zero pp, oct ou, positional sub-group u) of a tile: its bits, its value
 template <int GPW>
-__device__ __forceinline__ float tile_meta(const uint32_t (&m)[GPW], int ou, int u) {
+__device__ __forceinline__ uint32_t tile_meta_bits(const uint32_t (&m)[GPW], int ou, int u) {
     uint32_t word;
     bool hi;
     if (GPW == 1) {
@@ -53,7 +53,11 @@ __device__ __forceinline__ float tile_meta(const uint32_t (&m)[GPW], int ou, int
         word = (u & 2) ? m[(2 * ou + 1) % GPW] : m[(2 * ou) % GPW];
         hi = u & 1;
     }
-    return __half2float(__ushort_as_half(hi ? (uint16_t)(word >> 16) : (uint16_t)(word & 0xffffu)));
+    return hi ? word >> 16 : word & 0xffffu;
+}
+template <int GPW>
+__device__ __forceinline__ float tile_meta(const uint32_t (&m)[GPW], int ou, int u) {
+    return __half2float(__ushort_as_half((uint16_t)tile_meta_bits<GPW>(m, ou, u)));
 }
 
 // Byte tables of one (row, group): lo[h] / hi[h] hold the low / high bytes of the fp16 values of

@@ -885,8 +885,8 @@ static int launch_lut8_rows(int q, int gpw, const GemvArgs &a, dim3 grid, cudaSt
 // below the rounding of a 16-bit output; fp32 outputs therefore keep one row per pass and
 // fp32 entries, and so does the fused all-reduce.
 //
-// Plain launches of 3 <= m <= 16 rows at q = 2 or 3 with 16-bit outputs go to the small-batch kernel
-// instead (hlq_batch.cu: one pass over the weights for all rows; its weights are rounded to fp16,
+// Plain launches of 3 <= m <= 16 rows at q = 2, 3 or 4 with 16-bit outputs go to the small-batch kernel
+// instead (hlq_batch.cu: one pass over the weights for all rows; at 2 and 3 bits its weights are rounded to fp16,
 // which is below the rounding of a 16-bit output but not of an fp32 one), unless `lut_only` (a
 // weight whose extra bit-plane has already been added into accumulators of the LUT kernel's layout).
 static int launch_lut8_any(int q, int gpw, const GemvArgs &a_in, dim3 grid, cudaStream_t stream,
@@ -898,8 +898,8 @@ static int launch_lut8_any(int q, int gpw, const GemvArgs &a_in, dim3 grid, cuda
     if (!lut_only && !a.tp && !a.y_is_f32 && batch_mma_supported(q, m)) {
         // by measurement: the mma.sync kernel is the faster of the two at every m <= 16 (hlq_batch_umma.cu)
         const int which = g_batch_kernel.load(std::memory_order_relaxed);
-        if (which == 3 && a.use_rcodes && gpw == 1) return launch_batch_tmem(q, gpw, a, (int)grid.x, m, stream);
-        if (which == 2) return launch_batch_umma(q, gpw, a, (int)grid.x, m, stream);
+        if (which == 3 && a.use_rcodes && gpw == 1 && q < 4) return launch_batch_tmem(q, gpw, a, (int)grid.x, m, stream);
+        if (which == 2 && q < 4) return launch_batch_umma(q, gpw, a, (int)grid.x, m, stream);
         return launch_batch_mma(q, gpw, a, (int)grid.x, m, stream);
     }
     if (m < 2 || a.tp || a.y_is_f32) return launch_lut8_rows<1, false>(q, gpw, a, grid, stream);

@@ -61,6 +61,42 @@ def test_llama_shapes(L, n, k, q):
         assert O.normwise_error(forward(mod, x[:m]), ref[:m]) <= TOL_F16, m
 
 
+@pytest.mark.parametrize("g", [128, 64, 32])
+@pytest.mark.parametrize("n,k", [(200, 1152), (32, 512), (2080, 2560)])
+def test_four_planes_are_exact_up_to_the_output(L, n, k, g):
+    """3..16 rows at 4 bits: all operands of the products are exact, so what is left is the rounding of the
+    fp16 output (half an ulp, at most 2^-11 of the largest value) and that of the fp32 sums."""
+    d = O.synth_linear(n, k, 4, g, m=16, seed=41 + g, bias=True, signed_alpha=True)
+    mod = make(d, g, max_batch=16)
+    ref = O.hlq_linear(d["x"], d["w_quant"], d["w_scale"], d["w_zero"], g, d["bias"])
+    x = torch.from_numpy(d["x"]).cuda()
+    for m in (3, 4, 7, 8, 9, 13, 16):
+        assert O.normwise_error(forward(mod, x[:m]), ref[:m]) <= 2.0 ** -11 + 1e-5, m
+
+
+def test_group_finishes_blocks_between_segments(L):
+    """A group large enough that every CTA walks several segments, 4 bits and 9 rows: blocks finished in
+    the middle of a CTA's share are written and cleared, call after call."""
+    from elutq_b200 import linear
+    shapes = [(4096, 1024), (96, 2048), (8192, 512), (1000, 1536)]
+    data = [O.synth_linear(n, k, 4, 64, m=9, seed=77 + i) for i, (n, k) in enumerate(shapes * 4)]
+    weights = [linear.HLQWeight.from_export(F.ExportedLinear(d["w_quant"], d["w_scale"], d["w_zero"], d["bias"], 64), device=0)
+               for d in data]
+    xs = [torch.from_numpy(d["x"]).cuda() for d in data]
+    ys = [torch.full((9, n), -7.0, dtype=torch.float16, device="cuda") for n, _ in shapes * 4]
+    group = linear.HLQGroup(weights, max_m=16)
+    group.bind(xs, ys)
+    refs = [O.hlq_linear(d["x"], d["w_quant"], d["w_scale"], d["w_zero"], 64) for d in data]
+    for m in (9, 3, 9):
+        for y in ys:
+            y.fill_(-7.0)
+        group.forward(m)
+        assert group.kernel_status() == 0
+        for y, ref in zip(ys, refs):
+            assert O.normwise_error(y[:m].float().cpu().numpy().astype(np.float64), ref[:m]) <= 2.0 ** -11 + 1e-5
+            assert (y[m:] == -7.0).all()
+
+
 def test_repeated_calls_leave_clean_accumulators(L):
     """Calls with different row counts in a row: accumulators and counters return to zero each time, for
     this kernel's layout and the one-row kernel's alike."""

@@ -229,6 +229,28 @@ def test_pair_kernel_splits_a_long_k_over_the_pairs(built_lib, m):
         L.hlq_select_prefill_kernel(0)
 
 
+@pytest.mark.parametrize("q,n,k,g,m", [
+    (4, 250, 2048, 64, 17),       # n not a multiple of four: the finishing kernel one output a thread
+    (4, 1000, 1536, 32, 333),     # two token tiles of 192, K in parts
+    (3, 516, 4096, 128, 48),
+    (2, 256, 512, 64, 257),       # one slice: nothing to split
+    (1, 300, 2560, 128, 40),
+])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_tiles_and_parts_of_k(built_lib, q, n, k, g, m, dtype):
+    """The plan of tiles and parts of K over ragged sizes, every number of planes, calls back to back."""
+    d, mod = build(q, n, k, g, m, True, seed=900 + n + m)
+    x = torch.from_numpy(d["x"]).cuda().to(dtype)
+    ref = O.hlq_linear(x.float().cpu().numpy(), d["w_quant"], d["w_scale"], d["w_zero"], g, d["bias"])
+    outs = [mod(x) for _ in range(3)]
+    torch.cuda.synchronize()
+    assert mod.workspace.kernel_status() == 0
+    tol = TOL if dtype == torch.float16 else TOL_BF16_OUT
+    for y in outs:
+        assert O.normwise_error(y.float().cpu().numpy(), ref) <= tol
+        assert torch.equal(y, outs[0])
+
+
 @pytest.mark.parametrize("q,g", [(2, 64), (3, 128)])
 def test_random_sequence_of_calls_on_one_workspace(built_lib, q, g):
     """Forty calls with 1..300 rows, fp16 or bf16 inputs and every output type, in a seeded random
