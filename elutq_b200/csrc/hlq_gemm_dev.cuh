@@ -30,6 +30,7 @@ struct GemmArgs {
     int ksplit;          // pair kernel: parts K is split into (1: outputs are stored; > 1: sums go to acc)
     float *acc;          // pair kernel, ksplit > 1: ksplit fp32 slabs [m][n] in the workspace
     int y_dtype;
+    uint32_t table_entry_bytes;   // pair kernel: of a byte table
 };
 
 // programmatic dependent launch: the next kernel of the stream may start / everything before has finished

@@ -198,15 +198,22 @@ __device__ __forceinline__ void group_values(GroupValues<Q> &gv, const uint16_t 
         }
     }
 }
+// Entry of a byte table for byte k of a word.  The integer pipe is what the dequantizers wait for (80 % busy
+// in a product of few tokens), so the byte is brought down by one permute and the address formed by a
+// multiply: `entry`, the bytes of an entry, is an argument of the kernel because the compiler turns a
+// multiplication by a constant back into shifts on that pipe.
+template <typename T>
+__device__ __forceinline__ T table_entry(const unsigned char *tab, uint32_t word, int k, uint32_t entry) {
+    return *(const T *)(tab + __byte_perm(word, 0u, 0x4440u + k) * entry);
+}
 // 32 channels (bits[p] = the 32 bits of plane p in channel order) as 16 fp16 pairs
 template <int Q>
 __device__ __forceinline__ void expand32(const uint32_t (&bits)[Q], const GroupValues<Q> &gv, const unsigned char *tab,
-                                         uint32_t (&o)[16]) {
+                                         uint32_t entry, uint32_t (&o)[16]) {
     if constexpr (Q == 2) {
-        const uint2 *t = (const uint2 *)tab;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            const uint2 e0 = t[(bits[0] >> (8 * k)) & 0xffu], e1 = t[256 + ((bits[1] >> (8 * k)) & 0xffu)];
+            const uint2 e0 = table_entry<uint2>(tab, bits[0], k, entry), e1 = table_entry<uint2>(tab + 2048, bits[1], k, entry);
             const uint32_t sx = e0.x | e1.x, sy = e0.y | e1.y;
             o[4 * k] = prmt_b32(gv.v[0], gv.v[1], sx);
             o[4 * k + 1] = prmt_b32(gv.v[0], gv.v[1], sx >> 16);
@@ -214,12 +221,11 @@ __device__ __forceinline__ void expand32(const uint32_t (&bits)[Q], const GroupV
             o[4 * k + 3] = prmt_b32(gv.v[0], gv.v[1], sy >> 16);
         }
     } else {
-        const uint32_t *t = (const uint32_t *)tab;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            uint32_t code = t[(bits[0] >> (8 * k)) & 0xffu] | t[256 + ((bits[1] >> (8 * k)) & 0xffu)] |
-                            t[512 + ((bits[2] >> (8 * k)) & 0xffu)];
-            if constexpr (Q == 4) code |= t[768 + ((bits[Q - 1] >> (8 * k)) & 0xffu)];
+            uint32_t code = table_entry<uint32_t>(tab, bits[0], k, entry) | table_entry<uint32_t>(tab + 1024, bits[1], k, entry) |
+                            table_entry<uint32_t>(tab + 2048, bits[2], k, entry);
+            if constexpr (Q == 4) code |= table_entry<uint32_t>(tab + 3072, bits[Q - 1], k, entry);
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const uint32_t sel = h ? code >> 16 : code;
@@ -267,16 +273,22 @@ __device__ __forceinline__ void load_slice(RawSlice<Q> &rw, const GemmArgs &a, i
         }
     }
 }
-// the four words of a plane in source order: byte pair s of the lane's 16 bytes is stored at s ^ r
-__device__ __forceinline__ void source_words(const uint4 &w, int r, uint32_t (&o)[4]) {
-    uint32_t w0 = w.x, w1 = w.y, w2 = w.z, w3 = w.w, t;
-    if (r & 2) { t = w0; w0 = w1; w1 = t; t = w2; w2 = w3; w3 = t; }
-    if (r & 4) { t = w0; w0 = w2; w2 = t; t = w1; w1 = w3; w3 = t; }
-    if (r & 1) {
-        w0 = __funnelshift_l(w0, w0, 16); w1 = __funnelshift_l(w1, w1, 16);
-        w2 = __funnelshift_l(w2, w2, 16); w3 = __funnelshift_l(w3, w3, 16);
-    }
-    o[0] = w0; o[1] = w1; o[2] = w2; o[3] = w3;
+// The four words of a plane in source order: byte pair s of the lane's 16 bytes is stored at s ^ r.  Bit 2 of r
+// is a select between words two apart, bits 1 and 0 one permute over a pair of words.
+__device__ __forceinline__ uint32_t source_selector(int r) {
+    return (r & 2) ? ((r & 1) ? 0x5476u : 0x7654u) : ((r & 1) ? 0x1032u : 0x3210u);
+}
+__device__ __forceinline__ void source_words(const uint4 &w, bool far, uint32_t sel, uint32_t (&o)[4]) {
+    const uint32_t q0 = far ? w.z : w.x, q1 = far ? w.w : w.y, q2 = far ? w.x : w.z, q3 = far ? w.y : w.w;
+    o[0] = prmt_b32(q0, q1, sel);
+    o[1] = prmt_b32(q1, q0, sel);
+    o[2] = prmt_b32(q2, q3, sel);
+    o[3] = prmt_b32(q3, q2, sel);
+}
+// the fp16 scale or zero of stored group u among the four that a slice's fetch holds
+__device__ __forceinline__ uint16_t meta_of(const uint2 &m, int u) {
+    const uint32_t w = u & 2 ? m.y : m.x;
+    return (uint16_t)(u & 1 ? w >> 16 : w);
 }
 
 template <int Q>
@@ -539,6 +551,7 @@ dequant_gemm_pair_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap x
         bool ok = true;
         for (int u = pair; u < nunits && ok; u += npairs, ++it) {
             const int r = n & 7;
+            const uint32_t src_sel = source_selector(r);
             const int gsel = r >> a.gshift;      // stored group u holds source group u ^ gsel
             const int sl0 = unit_s0(u), sl1 = unit_s1(u);
             for (int sl = sl0; sl < sl1 && ok; ++sl, ++gs) {
@@ -553,7 +566,7 @@ dequant_gemm_pair_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap x
                 }
                 uint32_t src[Q][4];
 #pragma unroll
-                for (int p = 0; p < Q; ++p) source_words(cur.w[p], r, src[p]);
+                for (int p = 0; p < Q; ++p) source_words(cur.w[p], r & 4, src_sel, src[p]);
                 // K step 4 gs + part lives in stage `part`: the ring is one slice deep.  Half of the
                 // weights are made before the wait for the stage (it is busy for as long as the products
                 // that read it, and the arithmetic need not wait for them), the other half after.
@@ -571,12 +584,12 @@ dequant_gemm_pair_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap x
                     if (fresh || Q < 2) {
 #pragma unroll
                         for (int p = 0; p < Q; ++p)
-                            al[p] = (uint16_t)((((uint64_t)cur.mt[p].y << 32 | cur.mt[p].x) >> (16 * u)) & 0xffffu);
-                        z = (uint16_t)((((uint64_t)cur.mt[Q].y << 32 | cur.mt[Q].x) >> (16 * u)) & 0xffffu);
+                            al[p] = meta_of(cur.mt[p], u);
+                        z = meta_of(cur.mt[Q], u);
                     }
                     if constexpr (Q >= 2) {
                         if (fresh) group_values<Q>(gv, al, z);
-                        expand32<Q>(bits, gv, byte_tab, o);
+                        expand32<Q>(bits, gv, byte_tab, a.table_entry_bytes, o);
                     } else {
                         dequant_channels<Q, 32>(bits, al, z, lut, sel_lut, o);
                     }
@@ -766,6 +779,7 @@ int launch_dequant_gemm_pair(const GemmArgs &a_in, int q, const void *x, int sms
     if (!enc) return HLQ_ERR_NO_DEVICE;
     GemmArgs a = a_in;
     a.acc = acc;
+    a.table_entry_bytes = q == 2 ? 8 : 4;
     switch (q) {
         case 1: return launch_pair_inst<1>(a, x, enc, acc_bytes, stream);
         case 2: return launch_pair_inst<2>(a, x, enc, acc_bytes, stream);
