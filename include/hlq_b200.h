@@ -232,8 +232,9 @@ int hlq_workspace_status(const void *d_workspace, void *stream, int *kernel_stat
  * With HLQ_SHARD_COLS the result is this rank's partial sum.  Not re-entrant on one
  * workspace.  x and y must be 16-byte aligned.
  * Kernels by m (streaming layout): 1 or 2 rows, and fp32 outputs up to 16 rows: table-lookup
- * GEMV; 3..16 rows with 16-bit outputs at 2 or 3 bits: one pass over the weights for all rows
- * (dequantization in registers + mma.sync; the weights are rounded to fp16 there); more rows:
+ * GEMV; 3..16 rows with 16-bit outputs at 2 to 4 bits: one pass over the weights for all rows
+ * (dequantization in registers + mma.sync; 2- and 3-bit weights are rounded to fp16 there, 4-bit ones go
+ * in as one product per plane, unrounded); more rows:
  * dequantization + tcgen05 GEMM.
  * Replaces: arm_gemm, C++/ops/include/arm/arm_gemm.h:4-14 (dispatch at
  * C++/ops/src/arm/arm_gemm.cpp:871-924; GEMV worker :248-308, GEMM worker :362-387). */
@@ -254,7 +255,7 @@ int hlq_linear_forward_impl(int impl, int m, int k, int n, const void *d_x, int 
  * (correct, the slowest of the three), 3 = tcgen05.mma with the weight operand in tensor memory
  * (needs the row codes that hlq_weight_build_batch_codes makes for 2- and 3-bit weights with
  * g = 128 and rows a multiple of 128; other weights fall back to 1; as fast as 1 at 16 rows,
- * slower below).  Same results up to fp32 summation order. */
+ * slower below; 4-bit weights: always 1).  Same results up to fp32 summation order. */
 int hlq_select_batch_kernel(int which);
 
 /* Which kernel serves more than 16 rows of activations (for tests and measurements,
